@@ -34,11 +34,10 @@ constexpr int SST = UT + 4;  // row stride of the k-major operand tiles in share
 
 template <typename T>
 struct Dev {
-    const int32_t *ncol, *m, *c0, *idx_start, *idx, *relmap_start, *relmap, *uvec_start, *child_start, *child_list;
-    // per front row (offset idx_start[s] + k): the children's update-vector entries that land on it, child order
-    const int32_t *gat_start, *gat_src;
+    const int32_t *ncol, *m, *c0, *idx_start, *idx, *relmap_start, *relmap, *uvec_start;
+    const int32_t *gat_src;  // the children's update-vector entries that land on a front row (lists of three or more)
     const int64_t *front_off, *inv_off, *xinv_off;
-    T *F, *U, *Inv, *Xinv, *Abig;
+    T *F, *U, *Inv, *Xinv;
 };
 
 // Fronts at least this tall (and with more than kWideMinCols pivot columns) get a full pivot-block inverse and
@@ -527,48 +526,6 @@ static __global__ void k_xinv_reduce(Dev<T> D, const XTask *__restrict__ tasks, 
     }
 }
 
-// ---------------------------------------------------------------- solves of wide supernodes (batched multi-CTA GEMVs)
-// Per-front scratch vectors live at offset idx_start[s] (length m) in Abig (assembled right-hand side), Y1, Z.
-
-template <typename T>
-constexpr int kDotU = sizeof(T) == 4 ? 16 : 8;  // factor loads in flight per lane in the wide-front GEMVs
-
-// acc + sum of fa(c) fb(c) over c = first, first + G, .. < len (one lane's share of a dot product over G lanes). The
-// operands are loaded U at a time before any is used, so a lane keeps U loads in flight however short the run
-// (a plain strided loop waits out one memory latency per G elements); the products are added in the same order
-// as that loop's, so the sum is the same.
-template <int U, int G = 32, typename T, typename FA, typename FB>
-__device__ __forceinline__ T lane_dot(int first, int len, FA fa, FB fb, T acc)
-{
-    for (int c0 = first; c0 < len; c0 += G * U) {
-        T a[U], b[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int c = c0 + G * u;
-            a[u] = c < len ? fa(c) : T(0);
-            b[u] = c < len ? fb(c) : T(0);
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++)
-            if (c0 + G * u < len) acc = fma(a[u], b[u], acc);
-    }
-    return acc;
-}
-
-// acc = [b(cols); 0] - children's update vectors (in child order).
-template <typename T>
-__device__ __forceinline__ void dev_wide_acc(Dev<T> D, int s, const T *y, int chunk, int nchunk)
-{
-    int ms = D.m[s], nc = D.ncol[s], c0 = D.c0[s];
-    T *acc = D.Abig + D.idx_start[s];
-    const int32_t *gs = D.gat_start + D.idx_start[s];
-    for (int k = chunk * blockDim.x + threadIdx.x; k < ms; k += nchunk * blockDim.x) {
-        T v = k < nc ? y[c0 + k] : T(0);
-        for (int q = gs[k]; q < gs[k + 1]; q++) v -= D.U[D.gat_src[q]];
-        acc[k] = v;
-    }
-}
-
 // Mirror pass (end of a factorisation): every wide front's L21 is copied transposed into the front's unused upper
 // right block, F(k, nc + i) = L21(i, k), and its pivot-block inverse X into the unused upper triangle of its
 // storage, X(c, r) = X(r, c). The forward solve then reads a row of L21 or of X as one contiguous run (the same
@@ -628,143 +585,6 @@ static __global__ void __launch_bounds__(256) k_mirror(Dev<T> D, const int32_t *
         }
         __syncthreads();
     }
-}
-
-// One row of a mirrored operand against a vector: a dot product over a contiguous run by a group of G lanes
-// (G = 32: the whole warp; 16 or 8 for short rows, several rows to a warp), kDotU loads of each operand in flight
-// per lane, the group's lanes summed by a shuffle tree (fixed order). Every lane of the warp takes part in the
-// shuffles; a lane whose row does not exist passes len = 0.
-template <int G, typename T>
-__device__ __forceinline__ T group_dot(const T *__restrict__ row, const T *__restrict__ v, int len, int gl)
-{
-    T acc = lane_dot<kDotU<T>, G>(gl, len, [&](int c) { return row[c]; }, [&](int c) { return __ldg(v + c); }, T(0));
-    for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    return acc;
-}
-
-// Lanes per row (or column) of a wide front's pivot-block and L21 GEMVs whose rows have at most `len` entries.
-__host__ __device__ inline int fwd_group(int len) { return len <= 96 ? 8 : len <= 224 ? 16 : 32; }
-
-// Work lists of the wide fronts' solve kernels: per kind and level, (front, tile) pairs, a front's tiles in
-// order, the fronts of a level by descending pivot count. A CTA takes one pair, so no CTA of a launch is idle
-// however unequal the level's fronts.
-enum WideTileKind { kTileFwdY = 0, kTileFwdT = 1, kTileBwdX = 2, kTileBwdZ = 3, kTileAcc = 4, kTileKinds = 5 };
-
-// tiles of front (nc pivots, m rows) for each kind, for 512-thread CTAs
-__host__ __device__ inline int wide_tiles(int kind, int nc, int m)
-{
-    const int per = 16 * (32 / fwd_group(nc));
-    switch (kind) {
-    case kTileFwdY:
-    case kTileBwdX: return (nc + per - 1) / per;
-    case kTileFwdT: return (m - nc + per - 1) / per;
-    case kTileBwdZ: return (nc + 15) / 16;
-    default: return (m + 511) / 512;
-    }
-}
-
-// y1 = X acc1 (X lower triangular, read through its mirror: row r is X(c, r) for c <= r, contiguous), G lanes
-// per row, 16 * 32 / G rows per tile counted from the bottom (longest rows first)
-template <typename T, int G>
-__device__ __forceinline__ void dev_wide_fwd_y(Dev<T> D, int s, int tile, T *y, T *Y1)
-{
-    constexpr int RPC = 16 * (32 / G);
-    const int nc = D.ncol[s], c0 = D.c0[s], ntile = (nc + RPC - 1) / RPC;
-    if (tile >= ntile) return;
-    const int lane = threadIdx.x & 31, w0 = (ntile - 1 - tile) * RPC + (threadIdx.x >> 5) * (32 / G);
-    if (w0 >= nc) return;  // the warp's first row
-    const int r = w0 + lane / G;
-    const bool ok = r < nc;
-    const T v = group_dot<G>(D.Xinv + D.xinv_off[s] + (int64_t)(ok ? r : 0) * nc, D.Abig + D.idx_start[s],
-                             ok ? r + 1 : 0, lane % G);
-    if (ok && lane % G == 0) {
-        y[c0 + r] = v;
-        Y1[D.idx_start[s] + r] = v;
-    }
-}
-template <typename T>
-static __global__ void __launch_bounds__(512) k_wide_fwd_y(Dev<T> D, const int32_t *__restrict__ tiles, T *y, T *Y1)
-{
-    const int s = tiles[2 * blockIdx.x], tile = tiles[2 * blockIdx.x + 1], g = fwd_group(D.ncol[s]);
-    if (g == 8) dev_wide_fwd_y<T, 8>(D, s, tile, y, Y1);
-    else if (g == 16) dev_wide_fwd_y<T, 16>(D, s, tile, y, Y1);
-    else dev_wide_fwd_y<T, 32>(D, s, tile, y, Y1);
-}
-
-// update vector t = -acc2 + L21 y1 (L21 through its mirror: row i is F(k, nc + i), k < nc), G lanes per row,
-// 16 * 32 / G rows per tile
-template <typename T, int G>
-__device__ __forceinline__ void dev_wide_fwd_t(Dev<T> D, int s, int tile, const T *Y1)
-{
-    constexpr int RPC = 16 * (32 / G);
-    const int ms = D.m[s], nc = D.ncol[s], nr = ms - nc;
-    const int lane = threadIdx.x & 31, w0 = tile * RPC + (threadIdx.x >> 5) * (32 / G);
-    if (w0 >= nr) return;  // the warp's first row
-    const int i = w0 + lane / G;
-    const bool ok = i < nr;
-    const T v = group_dot<G>(D.F + D.front_off[s] + (int64_t)(nc + (ok ? i : 0)) * ms, Y1 + D.idx_start[s],
-                             ok ? nc : 0, lane % G);
-    if (ok && lane % G == 0) D.U[D.uvec_start[s] + i] = -D.Abig[D.idx_start[s] + nc + i] + v;
-}
-template <typename T>
-static __global__ void __launch_bounds__(512) k_wide_fwd_t(Dev<T> D, const int32_t *__restrict__ tiles, const T *Y1)
-{
-    const int s = tiles[2 * blockIdx.x], tile = tiles[2 * blockIdx.x + 1], g = fwd_group(D.ncol[s]);
-    if (g == 8) dev_wide_fwd_t<T, 8>(D, s, tile, Y1);
-    else if (g == 16) dev_wide_fwd_t<T, 16>(D, s, tile, Y1);
-    else dev_wide_fwd_t<T, 32>(D, s, tile, Y1);
-}
-
-// z = y1 - L21^T x2, one warp per pivot column; x2 is read through the front's row indices as the column
-// streams (the CTA's warps read the same entries, from L1), kDotU column loads in flight per lane.
-template <typename T>
-__device__ __forceinline__ void dev_wide_bwd_z(Dev<T> D, int s, int tile, const T *x, T *Z)
-{
-    int ms = D.m[s], nc = D.ncol[s], c0 = D.c0[s], nr = ms - nc;
-    int k = tile * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (k >= nc) return;
-    const int32_t *__restrict__ ix = D.idx + D.idx_start[s] + nc;
-    const T *__restrict__ col = D.F + D.front_off[s] + (int64_t)k * ms + nc;
-    int lane = threadIdx.x & 31;
-    T v = lane_dot<kDotU<T>>(lane, nr, [&](int i) { return col[i]; }, [&](int i) { return __ldg(x + __ldg(ix + i)); },
-                             T(0));
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) Z[D.idx_start[s] + k] = x[c0 + k] - v;
-}
-
-// x1 = X^T z, G lanes per pivot column j (column j of X is contiguous; G = 32 a warp, 16 or 8 for short columns,
-// several to a warp); z is staged in shared memory. Column group `tile` (16 * 32 / G columns) counted from the
-// right end (leftmost, longest columns first).
-template <typename T, int G>
-__device__ __forceinline__ void dev_wide_bwd_x(Dev<T> D, int s, int tile, const T *Z, T *x)
-{
-    extern __shared__ __align__(16) unsigned char zs_raw[];
-    T *zs = (T *)zs_raw;
-    constexpr int CPW = 32 / G;
-    int nc = D.ncol[s], c0 = D.c0[s];
-    int cpc = (blockDim.x >> 5) * CPW, nblk = (nc + cpc - 1) / cpc;
-    if (tile >= nblk) return;
-    int jbase = (nblk - 1 - tile) * cpc;
-    const T *z = Z + D.idx_start[s];
-    for (int i = jbase + threadIdx.x; i < nc; i += blockDim.x) zs[i - jbase] = z[i];
-    __syncthreads();
-    int lane = threadIdx.x & 31, jw = jbase + (threadIdx.x >> 5) * CPW;
-    if (jw >= nc) return;  // the warp's first column
-    int j = jw + lane / G;
-    const bool ok = j < nc;
-    const T *col = D.Xinv + D.xinv_off[s] + (int64_t)(ok ? j : 0) * nc;
-    T v = lane_dot<8, G>((ok ? j : nc) + lane % G, nc, [&](int i) { return col[i]; }, [&](int i) { return zs[i - jbase]; },
-                         T(0));
-    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (ok && lane % G == 0) x[c0 + j] = v;
-}
-template <typename T>
-static __global__ void __launch_bounds__(512) k_wide_bwd_x(Dev<T> D, const int32_t *__restrict__ tiles, const T *Z, T *x)
-{
-    const int s = tiles[2 * blockIdx.x], tile = tiles[2 * blockIdx.x + 1], g = fwd_group(D.ncol[s]);
-    if (g == 8) dev_wide_bwd_x<T, 8>(D, s, tile, Z, x);
-    else if (g == 16) dev_wide_bwd_x<T, 16>(D, s, tile, Z, x);
-    else dev_wide_bwd_x<T, 32>(D, s, tile, Z, x);
 }
 
 // Trailing update of every listed front by its pivot columns [k0, k0 + kd), kd = min(kdepth, ncol - k0):
@@ -1166,145 +986,6 @@ static __global__ void k_init_err(int *err)
     err[2] = 0;
 }
 
-template <typename T>
-static __global__ void k_permute_in(int n, const int32_t *perm, const double *b, T *y)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) y[i] = (T)b[perm[i]];
-}
-template <typename T>
-static __global__ void k_permute_out(int n, const int32_t *perm, const T *y, double *x)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) x[perm[i]] = (double)y[i];
-}
-
-// Forward elimination of the fronts of one level: y(cols) and the update vector for the parent. Each 64-pivot
-// block is applied through its stored inverse (one block GEMV) instead of 64 dependent steps.
-template <typename T>
-__device__ __forceinline__ void dev_forward(Dev<T> D, int s, T *y)
-{
-    extern __shared__ __align__(16) unsigned char acc_raw[];
-    T *acc = (T *)acc_raw;
-    __shared__ T yb[PW];
-    int ms = D.m[s], nc = D.ncol[s], c0 = D.c0[s];
-    const T *F = D.F + D.front_off[s];
-    const T *Inv = D.Inv + D.inv_off[s];
-    int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-    const int32_t *gs = D.gat_start + D.idx_start[s];
-    for (int k = tid; k < ms; k += nt) {
-        T v = k < nc ? y[c0 + k] : T(0);
-        for (int q = gs[k]; q < gs[k + 1]; q++) v -= D.U[D.gat_src[q]];
-        acc[k] = v;
-    }
-    __syncthreads();
-    for (int kb = 0; kb < nc; kb += PW) {
-        int w = min(PW, nc - kb);
-        const T *I = Inv + (int64_t)(kb / PW) * PW * PW;
-        // y_blk = Linv acc_blk (warp per output row, coalesced over the inverse's columns? rows: I[c*PW + i])
-        for (int i = warp; i < w; i += nw) {
-            T v = lane_dot<2>(lane, i + 1, [&](int c) { return I[(int64_t)c * PW + i]; }, [&](int c) { return acc[kb + c]; },
-                              T(0));
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) yb[i] = v;
-        }
-        __syncthreads();
-        for (int i = tid; i < w; i += nt) acc[kb + i] = yb[i];
-        // rows below the block
-        for (int r = kb + w + tid; r < ms; r += nt) {
-            T v = acc[r];
-            // the block's w <= 64 entries of row r, 16 loads in flight
-            for (int k0 = 0; k0 < w; k0 += 16) {
-                T f[16];
-#pragma unroll
-                for (int u = 0; u < 16; u++) f[u] = k0 + u < w ? F[(int64_t)(kb + k0 + u) * ms + r] : T(0);
-#pragma unroll
-                for (int u = 0; u < 16; u++)
-                    if (k0 + u < w) v = fma(-f[u], yb[k0 + u], v);
-            }
-            acc[r] = v;
-        }
-        __syncthreads();
-    }
-    for (int k = tid; k < nc; k += nt) y[c0 + k] = acc[k];
-    T *u = D.U + D.uvec_start[s];
-    for (int i = tid; i < ms - nc; i += nt) u[i] = -acc[nc + i];
-}
-
-// Back substitution of the fronts of one level: x(cols) from y(cols) and the solved ancestors' x.
-template <typename T>
-__device__ __forceinline__ void dev_backward(Dev<T> D, int s, const T *y, T *x)
-{
-    extern __shared__ __align__(16) unsigned char sm_raw[];
-    T *sm = (T *)sm_raw;
-    __shared__ T xb[PW];
-    int ms = D.m[s], nc = D.ncol[s], c0 = D.c0[s], nr = ms - nc;
-    const T *F = D.F + D.front_off[s];
-    const T *Inv = D.Inv + D.inv_off[s];
-    const int32_t *ix = D.idx + D.idx_start[s];
-    T *acc = sm, *xs = sm + nc;
-    int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-    for (int k = tid; k < nc; k += nt) acc[k] = y[c0 + k];
-    for (int i = tid; i < nr; i += nt) xs[i] = x[ix[nc + i]];
-    __syncthreads();
-    for (int k = warp; k < nc; k += nw) {
-        const T *col = F + (int64_t)k * ms + nc;
-        T v = lane_dot<8>(lane, nr, [&](int i) { return col[i]; }, [&](int i) { return xs[i]; }, T(0));
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) acc[k] -= v;
-    }
-    __syncthreads();
-    int nblk = (nc + PW - 1) / PW;
-    for (int bi = nblk - 1; bi >= 0; bi--) {
-        int kb = bi * PW, w = min(PW, nc - kb), ke = kb + w;
-        for (int j = kb + warp; j < ke; j += nw) {
-            const T *col = F + (int64_t)j * ms;
-            T v = lane_dot<8>(ke + lane, nc, [&](int k) { return col[k]; }, [&](int k) { return acc[k]; }, T(0));
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) acc[j] -= v;
-        }
-        __syncthreads();
-        // x_blk = Linv^T acc_blk: x_j = sum_{i >= j} Linv[i][j] acc_i (column j of the inverse is contiguous)
-        const T *I = Inv + (int64_t)bi * PW * PW;
-        for (int j = warp; j < w; j += nw) {
-            T v = lane_dot<2>(j + lane, w, [&](int i) { return I[(int64_t)j * PW + i]; }, [&](int i) { return acc[kb + i]; },
-                              T(0));
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (lane == 0) xb[j] = v;
-        }
-        __syncthreads();
-        for (int j = tid; j < w; j += nt) acc[kb + j] = xb[j];
-        __syncthreads();
-    }
-    for (int k = tid; k < nc; k += nt) x[c0 + k] = acc[k];
-}
-
-// One launch per level and sweep direction covers both kinds of front: the small fronts (one CTA each, whole
-// elimination) and the first phase of the wide ones (the assembled right-hand side going up, z = y1 - L21^T x2
-// coming down).
-template <typename T>
-static __global__ void __launch_bounds__(512) k_fwd_level(Dev<T> D, const int32_t *__restrict__ small, int nsmall,
-                                                          const int32_t *__restrict__ tiles, T *y)
-{
-    if ((int)blockIdx.x < nsmall) {
-        dev_forward(D, small[blockIdx.x], y);
-    } else {
-        // a wide front's rows are shared by ceil(m / 512) CTAs, one tile each
-        const int t = blockIdx.x - nsmall, s = tiles[2 * t];
-        dev_wide_acc(D, s, y, tiles[2 * t + 1], (D.m[s] + blockDim.x - 1) / blockDim.x);
-    }
-}
-
-template <typename T>
-static __global__ void __launch_bounds__(512) k_bwd_level(Dev<T> D, const int32_t *__restrict__ small, int nsmall,
-                                                          const int32_t *__restrict__ tiles, T *x, T *Z)
-{
-    if ((int)blockIdx.x < nsmall) {
-        dev_backward(D, small[blockIdx.x], x, x);
-    } else {
-        const int t = blockIdx.x - nsmall;
-        dev_wide_bwd_z(D, tiles[2 * t], tiles[2 * t + 1], x, Z);
-    }
-}
-
 static __global__ void k_finite(int n, const double *x, int *flag)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -1312,6 +993,11 @@ static __global__ void k_finite(int n, const double *x, int *flag)
 }
 
 }  // namespace mf
+}  // namespace ifea
+
+#include "sweep.cuh"
+
+namespace ifea {
 
 // The linear solver behind the stepper: analyse once per pattern, factorise device values, solve on the device.
 // Implemented by the multifrontal Cholesky in double precision (the drop-in) and in single precision (the factor
@@ -1340,7 +1026,7 @@ public:
     virtual int value_bytes() const = 0;
     virtual int64_t tc_launches() const = 0;  // tensor-core trailing-update launches in one factorisation
     virtual void set_tc(bool on, int rows) = 0;  // tensor-core trailing updates (single precision) from `rows` rows
-    // host seconds spent in: 0 symbolic analysis, 1 its device tables, 2 the factorisation graph, 3 the solve graph
+    // host seconds spent in: 0 symbolic analysis, 1 its device tables, 2 the factorisation graph, 3 unused
     virtual double setup_s(int part) const = 0;
 };
 
@@ -1366,6 +1052,7 @@ public:
         cusparseSetMatType(descr_, CUSPARSE_MATRIX_TYPE_GENERAL);
         cusparseSetMatIndexBase(descr_, CUSPARSE_INDEX_BASE_ZERO);
         d_err_.resize(4);
+        d_err_.zero(st_);
         cuda_check(cudaStreamCreateWithFlags(&cap_, cudaStreamNonBlocking), "cudaStreamCreate");
         cuda_check(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "cudaStreamCreate");
         cuda_check(cudaStreamCreateWithFlags(&ahead_, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -1466,8 +1153,6 @@ public:
             for (int s = 0; s < S.nsuper; s++)
                 if (S.parent[s] >= 0) cl[fill[S.parent[s]]++] = s;
         }
-        d_cs_.upload(cs, st_);
-        d_cl_.upload(cl, st_);
         {
             // gather lists: for every front row, its children's update entries in child order (the order the
             // extend-add of the solves applies them in)
@@ -1487,7 +1172,9 @@ public:
                     for (int i = 0; i < nr; i++)
                         gsrc[fill[S.idx_start[p] + S.relmap[S.relmap_start[c] + i]]++] = S.uvec_start[c] + i;
                 }
-            d_gst_.upload(gst, st_);
+            std::vector<int2> pair;
+            mf::sweep_pairs(gst, gsrc, pair);
+            d_pair_.upload(pair, st_);
             d_gsrc_.upload(gsrc, st_);
         }
         // per level: fronts sorted by pivot count (descending) so each panel step's active fronts are a prefix
@@ -1517,7 +1204,8 @@ public:
             big_start_[l] = (int32_t)big_list_.size();
             for (int32_t q = S.level_start[l]; q < S.level_start[l + 1]; q++) {
                 int sn = S.level_list[q];
-                if (S.m[sn] >= wide_m_ && S.ncol[sn] > mf::kWideMinCols) {
+                // (a front taller than one CTA's shared memory is wide whatever the bound)
+                if ((S.m[sn] >= wide_m_ && S.ncol[sn] > mf::kWideMinCols) || S.m[sn] * sizeof(T) > 128 * 1024) {
                     big_list_.push_back(sn);
                     xinv_off_[sn] = xinv_total;
                     xinv_total += (int64_t)S.ncol[sn] * S.ncol[sn];
@@ -1534,27 +1222,6 @@ public:
                              [&](int a, int b) { return S.ncol[a] > S.ncol[b]; });
         d_big_.upload(big_list_, st_);
         {
-            // the solve kernels' work lists (pairs (front, tile), kinds x levels)
-            const int nl1 = S.nlevels + 1;
-            std::vector<int32_t> wt;
-            wt_start_.assign(mf::kTileKinds * nl1, 0);
-            for (int kind = 0; kind < mf::kTileKinds; kind++) {
-                for (int l = 0; l < S.nlevels; l++) {
-                    wt_start_[kind * nl1 + l] = (int32_t)(wt.size() / 2);
-                    for (int q = big_start_[l]; q < big_start_[l + 1]; q++) {
-                        const int sn = big_list_[q], nt = mf::wide_tiles(kind, S.ncol[sn], S.m[sn]);
-                        for (int t = 0; t < nt; t++) {
-                            wt.push_back(sn);
-                            wt.push_back(t);
-                        }
-                    }
-                }
-                wt_start_[kind * nl1 + S.nlevels] = (int32_t)(wt.size() / 2);
-            }
-            if (wt.empty()) wt.assign(2, 0);
-            d_wtiles_.upload(wt, st_);
-        }
-        {
             std::vector<int64_t> ts(big_list_.size() + 1, 0);
             for (size_t q = 0; q < big_list_.size(); q++) {
                 int sn = big_list_[q], nc = S.ncol[sn], nr = S.m[sn] - nc, tk = (nc + 31) / 32, tr = (nr + 31) / 32;
@@ -1563,10 +1230,9 @@ public:
             mirror_tiles_ = ts.back();
             d_mirror_ts_.upload(ts, st_);
         }
-        wide_smem_ = 8;
-        for (int sn : big_list_) wide_smem_ = std::max(wide_smem_, (size_t)std::max(S.ncol[sn], S.m[sn] - S.ncol[sn]) * sizeof(T));
-        if (wide_smem_ > 200 * 1024) throw Failure(IFEA_INPUT_INVALID, "front larger than the wide solve kernels' shared-memory window");
-        ensure_dynamic_smem((const void *)mf::k_wide_bwd_x<T>, (int)wide_smem_);
+        for (int sn : big_list_)
+            if ((size_t)std::max(S.ncol[sn], S.m[sn] - S.ncol[sn]) * sizeof(T) > 200 * 1024)
+                throw Failure(IFEA_INPUT_INVALID, "front larger than the wide solve kernels' shared-memory window");
         // inverse passes of the wide supernodes, per level: diagonal copies, then for groups of 2, 4, ... blocks
         // the T pass and the X21 pass, each followed by its reduction when a block range was split
         std::vector<mf::XTask> tasks;
@@ -1628,18 +1294,13 @@ public:
         d_xinv_off_.upload(xinv_off_, st_);
         d_Xinv_.resize(std::max<int64_t>(xinv_total, 1));
         d_Abig_.resize(S.idx_start[S.nsuper]);
-        d_y1_.resize(S.idx_start[S.nsuper]);
-        d_z_.resize(S.idx_start[S.nsuper]);
-        small_smem_ = (size_t)max_small_m * sizeof(T);
         d_F_.resize(S.pool);
         d_U_.resize(std::max<int64_t>(S.uvec_pool, 1));
-        d_y_.resize(S.n);
+        d_y_.resize(3 * (size_t)S.n);
         dev_.ncol = d_ncol_; dev_.m = d_m_; dev_.c0 = d_c0_; dev_.idx_start = d_idxs_; dev_.idx = d_idx_;
-        dev_.relmap_start = d_rms_; dev_.relmap = d_rm_; dev_.uvec_start = d_uvs_; dev_.child_start = d_cs_;
-        dev_.child_list = d_cl_; dev_.front_off = d_off_; dev_.F = d_F_; dev_.U = d_U_;
-        dev_.gat_start = d_gst_; dev_.gat_src = d_gsrc_;
+        dev_.relmap_start = d_rms_; dev_.relmap = d_rm_; dev_.uvec_start = d_uvs_; dev_.front_off = d_off_; dev_.F = d_F_; dev_.U = d_U_;
+        dev_.gat_src = d_gsrc_;
         dev_.inv_off = d_inv_off_; dev_.Inv = d_Inv_; dev_.xinv_off = d_xinv_off_; dev_.Xinv = d_Xinv_;
-        dev_.Abig = d_Abig_;
         ensure_dynamic_smem((const void *)mf::k_update<T>, (int)kUpdateSmem);
         if constexpr (std::is_same<T, float>::value)
             ensure_dynamic_smem((const void *)mf::k_update_sp, mf::tcu::kSmem);
@@ -1647,10 +1308,22 @@ public:
         ensure_dynamic_smem((const void *)mf::k_panel_trsm<T>, (int)kPairSmem);
         ensure_dynamic_smem((const void *)mf::k_xinv_gemm<T, 0>, (int)kPairSmem);
         ensure_dynamic_smem((const void *)mf::k_xinv_gemm<T, 1>, (int)kPairSmem);
-        if (small_smem_ > 200 * 1024) throw Failure(IFEA_INPUT_INVALID, "front larger than the solve kernels' shared-memory window");
-        level_smem_ = small_smem_;  // the wide fronts' z pass stages nothing
-        ensure_dynamic_smem((const void *)mf::k_fwd_level<T>, (int)small_smem_);
-        ensure_dynamic_smem((const void *)mf::k_bwd_level<T>, (int)level_smem_);
+        const size_t small_smem = (size_t)max_small_m * sizeof(T);
+        if (small_smem > 200 * 1024) throw Failure(IFEA_INPUT_INVALID, "front larger than the solve kernels' shared-memory window");
+        {
+            std::vector<mf::SweepTask> tasks;
+            int vec = 1, width = 1, per_sm = 1;
+            mf::sweep_tasks<T>(S, small_start_, small_list_, big_start_, big_list_, inv_off_, xinv_off_, tasks, vec, width);
+            d_sweep_.upload(tasks, st_);
+            sweep_smem_ = std::max(small_smem, (size_t)vec * sizeof(T));
+            ensure_dynamic_smem((const void *)mf::k_sweep<T>, (int)sweep_smem_);
+            cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mf::k_sweep<T>, mf::kSwThreads, sweep_smem_), "occupancy");
+            // no more CTAs than the widest phase has tiles (and some to wait for the next one)
+            sweep_grid_ = std::max(1, std::min(148 * std::max(1, per_sm), width + width / 2));
+            d_cnt_.resize((size_t)mf::kCntN * S.nsuper + 1);
+            d_cnt_.zero(st_);
+            sweep_epoch_ = 0;
+        }
         cuda_check(cudaStreamSynchronize(st_), "cudaStreamSynchronize");
         analyzed_ = true;
     }
@@ -1679,12 +1352,13 @@ public:
         cuda_check(cudaEventRecord(ev_[0], st_), "cudaEventRecord");
         cuda_check(cudaGraphLaunch(factor_exec_, st_), "cudaGraphLaunch");
         cuda_check(cudaEventRecord(ev_[1], st_), "cudaEventRecord");
-        int32_t e[3];
+        int32_t e[4];
         cuda_check(cudaMemcpyAsync(e, d_err_.p, sizeof e, cudaMemcpyDeviceToHost, st_), "D2H");
         cuda_check(cudaStreamSynchronize(st_), "cudaStreamSynchronize");
         float ms = 0;
         if (cudaEventElapsedTime(&ms, ev_[0], ev_[1]) == cudaSuccess) factor_ms_ += ms;
         if (e[2]) throw Failure(IFEA_CUDA_ERROR, "multifrontal factorisation: a tensor-core update timed out");
+        if (e[3]) abandoned();
         if (e[0] != INT_MAX) {
             int row = S.perm[e[0]];
             throw Failure(IFEA_NOT_SPD, "Stiffness matrix not positive definite at equation " + std::to_string(row) +
@@ -1891,27 +1565,31 @@ public:
         cuda_check(cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...), "cudaLaunchKernelEx");
     }
 
-    // x = A^-1 b on the device (b and x may alias). The level sweeps run as one captured CUDA graph on the
-    // solver's internal vector; only the permutations in and out are launched per call.
+    // x = A^-1 b on the device (b and x may alias: an entry of x is written after every read of b in its tree).
     void solve(const double *d_b, double *d_x) override
     {
         if (!factored_) throw Failure(IFEA_BAD_STATE, "Factorize must be called first.");
         const MfSymbolic &S = sym_;
-        int n = S.n, g = std::max(1, std::min((n + 255) / 256, 4 * 148));
-        if (!solve_exec_) {
-            HostClock hc(setup_s_[3]);
-            cudaGraph_t gr = nullptr;
-            cuda_check(cudaStreamBeginCapture(cap_, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-            enqueue_sweeps(cap_);
-            cuda_check(cudaStreamEndCapture(cap_, &gr), "cudaStreamEndCapture");
-            cudaError_t e = cudaGraphInstantiate(&solve_exec_, gr, 0);
-            cudaGraphDestroy(gr);
-            cuda_check(e, "cudaGraphInstantiate");
-        }
+        mf::SweepArgs<T> a;
+        a.D = dev_;
+        a.tasks = d_sweep_.p;
+        a.ntasks = (int)d_sweep_.n;
+        a.cnt = d_cnt_.p;
+        a.ticket = d_cnt_.p + (size_t)mf::kCntN * S.nsuper;
+        a.ticket0 = sweep_epoch_ * (uint32_t)(a.ntasks + sweep_grid_);  // every CTA draws one ticket past the list
+        a.epoch = ++sweep_epoch_;
+        a.perm = d_perm_;
+        a.pair = d_pair_.p;
+        a.b = d_b;
+        a.x = d_x;
+        a.A1 = d_Abig_;
+        a.Y = d_y_.p;
+        a.Z = d_y_.p + S.n;
+        a.X = d_y_.p + 2 * (size_t)S.n;
+        a.err = d_err_.p + 3;
+        a.n = S.n;
         if (profile_) cuda_check(cudaEventRecord(ev_[2], st_), "cudaEventRecord");
-        mf::k_permute_in<T><<<g, 256, 0, st_>>>(n, d_perm_, d_b, d_y_);
-        cuda_check(cudaGraphLaunch(solve_exec_, st_), "cudaGraphLaunch");
-        mf::k_permute_out<T><<<g, 256, 0, st_>>>(n, d_perm_, d_y_, d_x);
+        mf::k_sweep<T><<<sweep_grid_, mf::kSwThreads, sweep_smem_, st_>>>(a);
         n_solves_++;
         if (profile_) {
             cuda_check(cudaEventRecord(ev_[3], st_), "cudaEventRecord");
@@ -1922,52 +1600,30 @@ public:
         cuda_check(cudaGetLastError(), "multifrontal solve launch");
     }
 
-    void enqueue_sweeps(cudaStream_t st)
-    {
-        const MfSymbolic &S = sym_;
-        const int nl1 = S.nlevels + 1;
-        // pairs [first, first + count) of kind k at level l in the work lists
-        auto tiles = [&](int k, int l, int &count) {
-            count = wt_start_[k * nl1 + l + 1] - wt_start_[k * nl1 + l];
-            return d_wtiles_.p + 2 * (int64_t)wt_start_[k * nl1 + l];
-        };
-        int n;
-        for (int l = 0; l < S.nlevels; l++) {
-            int q0 = small_start_[l], cnt = small_start_[l + 1] - q0;
-            const int32_t *acc = tiles(mf::kTileAcc, l, n);
-            if (cnt + n > 0)
-                mf::k_fwd_level<T><<<cnt + n, 512, small_smem_, st>>>(dev_, d_small_.p + q0, cnt, acc, d_y_);
-            const int32_t *ty = tiles(mf::kTileFwdY, l, n);
-            if (n > 0) mf::k_wide_fwd_y<T><<<n, 512, 0, st>>>(dev_, ty, d_y_, d_y1_);
-            const int32_t *tt = tiles(mf::kTileFwdT, l, n);
-            if (n > 0) mf::k_wide_fwd_t<T><<<n, 512, 0, st>>>(dev_, tt, d_y1_);
-        }
-        for (int l = S.nlevels - 1; l >= 0; l--) {
-            int q0 = small_start_[l], cnt = small_start_[l + 1] - q0;
-            const int32_t *tz = tiles(mf::kTileBwdZ, l, n);
-            if (cnt + n > 0)
-                mf::k_bwd_level<T><<<cnt + n, 512, level_smem_, st>>>(dev_, d_small_.p + q0, cnt, tz, d_y_, d_z_);
-            const int32_t *tx = tiles(mf::kTileBwdX, l, n);
-            if (n > 0) mf::k_wide_bwd_x<T><<<n, 512, wide_smem_, st>>>(dev_, tx, d_z_, d_y_);
-        }
-    }
-
     void check_finite(const double *d_x) override
     {
-        int32_t zero = 0, f = 0;
+        int32_t zero = 0, f[3] = {0, 0, 0};
         cuda_check(cudaMemcpyAsync(d_err_.p + 1, &zero, sizeof zero, cudaMemcpyHostToDevice, st_), "H2D");
         mf::k_finite<<<std::max(1, std::min((sym_.n + 255) / 256, 592)), 256, 0, st_>>>(sym_.n, d_x, d_err_.p + 1);
-        cuda_check(cudaMemcpyAsync(&f, d_err_.p + 1, sizeof f, cudaMemcpyDeviceToHost, st_), "D2H");
+        cuda_check(cudaMemcpyAsync(f, d_err_.p + 1, sizeof f, cudaMemcpyDeviceToHost, st_), "D2H");
         cuda_check(cudaStreamSynchronize(st_), "cudaStreamSynchronize");
-        if (f) throw Failure(IFEA_NOT_SPD, "Stiffness matrix not positive definite at equation -1 (pivot NaN).");
+        if (f[2]) abandoned();
+        if (f[0]) throw Failure(IFEA_NOT_SPD, "Stiffness matrix not positive definite at equation -1 (pivot NaN).");
     }
 
 private:
+    // a sweep gave up waiting: its counters are not usable any more
+    void abandoned()
+    {
+        d_err_.zero(st_);
+        d_cnt_.zero(st_);
+        sweep_epoch_ = 0;
+        throw Failure(IFEA_CUDA_ERROR, "multifrontal solve: a wait for another tile timed out");
+    }
     void drop_graphs()
     {
-        if (solve_exec_) cudaGraphExecDestroy(solve_exec_);
         if (factor_exec_) cudaGraphExecDestroy(factor_exec_);
-        solve_exec_ = factor_exec_ = nullptr;
+        factor_exec_ = nullptr;
         factor_vals_ = nullptr;
     }
     cudaEvent_t ev_[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -1988,7 +1644,7 @@ private:
     int prio_hi_ = 0;  // greatest stream priority of the device
     std::vector<cudaEvent_t> fork_ev_;
     cudaEvent_t join_ev_ = nullptr;
-    cudaGraphExec_t solve_exec_ = nullptr, factor_exec_ = nullptr;
+    cudaGraphExec_t factor_exec_ = nullptr;
     const double *factor_vals_ = nullptr;
     static constexpr size_t kUpdateSmem = 2 * mf::PW * mf::SST * sizeof(T);
     static constexpr size_t kPairSmem = 2 * mf::PW * mf::SST * sizeof(T);
@@ -1997,23 +1653,26 @@ private:
     cusolverSpHandle_t hsp_ = nullptr;
     std::vector<int64_t> inv_off_, xinv_off_;
     std::vector<int32_t> small_start_, small_list_, big_start_, big_list_;
-    std::vector<int32_t> wt_start_;  // work-list offsets of the wide solve kernels, kind x (levels + 1)
+    DBuf<mf::SweepTask> d_sweep_;   // the solve's task list
+    DBuf<uint32_t> d_cnt_;          // its completion counters, then the ticket
+    uint32_t sweep_epoch_ = 0;      // solves since the counters were cleared
+    int sweep_grid_ = 1;
     std::vector<int> xinv_pass_start_, xinv_task_start_, xinv_pass_kind_;
     DBuf<mf::XTask> d_xinv_tasks_;
     DBuf<T> d_xinv_w_;
     static constexpr int kXinvChunk = 4;  // tile steps per CTA before a block range is split
-    size_t small_smem_ = 8, wide_smem_ = 8, level_smem_ = 8;
+    size_t sweep_smem_ = 8;
     DBuf<int64_t> d_inv_off_, d_xinv_off_;
     DBuf<int64_t> d_mirror_ts_;   // the wide fronts' mirror tiles, prefix per front
     int64_t mirror_tiles_ = 0;
-    DBuf<int32_t> d_small_, d_big_, d_gst_, d_gsrc_, d_wtiles_;
-    DBuf<T> d_Inv_, d_Xinv_, d_Abig_, d_y1_, d_z_;
+    DBuf<int32_t> d_small_, d_big_, d_gsrc_;
+    DBuf<int2> d_pair_;
+    DBuf<T> d_Inv_, d_Xinv_, d_Abig_;
     cusparseMatDescr_t descr_ = nullptr;
     MfSymbolic sym_;
     bool analyzed_ = false, factored_ = false;
     std::vector<int32_t> lvl_sorted_;
-    DBuf<int32_t> d_ncol_, d_m_, d_c0_, d_idxs_, d_idx_, d_rms_, d_rm_, d_uvs_, d_par_, d_perm_, d_asrc_, d_ext_, d_cs_,
-        d_cl_, d_lvl_, d_err_;
+    DBuf<int32_t> d_ncol_, d_m_, d_c0_, d_idxs_, d_idx_, d_rms_, d_rm_, d_uvs_, d_par_, d_perm_, d_asrc_, d_ext_, d_lvl_, d_err_;
     DBuf<int64_t> d_off_, d_adst_;
     DBuf<T> d_F_, d_U_, d_y_;
     mf::Dev<T> dev_{};
