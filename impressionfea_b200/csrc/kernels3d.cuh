@@ -64,6 +64,12 @@ __device__ __forceinline__ double quality_of(const View3 &V, const double *x, in
     return tet_quality(ld3(x, t[0]), ld3(x, t[1]), ld3(x, t[2]), ld3(x, t[3]));
 }
 
+// Workspace of the conjugate gradients: partial sums and arrival ticket of one kernel's dot product, convergence flag.
+struct PcgWork {
+    double *part;
+    int32_t *ticket, *stop;
+};
+
 #define GRID_STRIDE(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 
 // Writes the block's K partial sums to partials[slot_k][blockIdx.x].
@@ -568,9 +574,38 @@ __global__ void k_regularise(View3 V)
     }
 }
 
-// y = A x with A the assembled values in 3x3 node blocks, row form: one warp per node.
-__global__ void k_spmv(View3 V, const double *__restrict__ x, double *__restrict__ y)
+// Sums K values over the grid in one launch: every block leaves its partial sums, the last block to arrive (whichever
+// that is) adds them in block order, so the result does not depend on the order of arrival. True in the last block,
+// whose thread 0 holds the sums. part: K x gridDim.x doubles; ticket: zero, and zero again afterwards.
+template <int K>
+__device__ __forceinline__ bool grid_sum(double (&acc)[K], double *part, int32_t *ticket)
 {
+    __shared__ double sh[32 * K];
+    __shared__ bool last;
+    block_sum<K>(acc, sh);
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < K; k++) part[k * gridDim.x + blockIdx.x] = acc[k];
+        __threadfence();
+        last = atomicAdd(ticket, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    for (int k = 0; k < K; k++) {
+        acc[k] = 0;
+        for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) acc[k] += __ldcg(part + k * gridDim.x + i);
+    }
+    block_sum<K>(acc, sh);
+    if (threadIdx.x == 0) *ticket = 0;
+    return true;
+}
+
+// y = A x with A the assembled values in 3x3 node blocks, row form: one warp per node; with W.part also
+// scalars[S_PQ] = x.y (the conjugate gradients' step length).
+__global__ void k_spmv(View3 V, const double *__restrict__ x, double *__restrict__ y, PcgWork W)
+{
+    if (W.stop && *W.stop) return;
+    double xy[1] = {0};
     int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     int nw = (gridDim.x * blockDim.x) >> 5;
     for (int j = warp; j < V.nn; j += nw) {
@@ -584,8 +619,12 @@ __global__ void k_spmv(View3 V, const double *__restrict__ x, double *__restrict
         }
         for (int ci = 0; ci < 3; ci++)
             for (int o = 16; o > 0; o >>= 1) s[ci] += __shfl_xor_sync(0xffffffffu, s[ci], o);
-        if (lane < 3) y[3 * j + lane] = s[lane];
+        if (lane < 3) {
+            y[3 * j + lane] = s[lane];
+            xy[0] += s[lane] * x[3 * j + lane];
+        }
     }
+    if (W.part && grid_sum<1>(xy, W.part, W.ticket) && threadIdx.x == 0) V.scalars[S_PQ] = xy[0];
 }
 
 // partials: slot A = sum a.b, slot B = sum a.a (optional)
@@ -1016,24 +1055,54 @@ __global__ void k_initial_velocity(View3 V, double rate_ref, double cx, double c
 }  // namespace ifea
 
 namespace ifea {
-// PCG pieces with the step scalars kept on the device (Pcg, Forging3DSolver.cs:1051-1087).
-__global__ void k_pcg_residual(int n, const double *b, const double *q, double *r)
+// PCG pieces with the step scalars and the convergence test kept on the device (Pcg, Forging3DSolver.cs:1051-1087):
+// five launches an iteration (product and p.q; x, r and |r|^2; the factor's solve; r.z; p) where the dot products, their
+// final sums and the roll of r.z took ten, and nothing of an iteration does anything once *stop is set, so the host
+// may run one iteration ahead of the residual it reads. The launches are bound by their own fixed cost (2-3 us each
+// at 5k-30k tets).
+// r = b - q (q = A x), or x += alpha p, r -= alpha q; then scalars[S_RR] = r.r and whether the iteration has converged.
+__global__ void k_pcg_residual(View3 V, double tol, const double *b, const double *q, double *r, PcgWork W)
 {
-    GRID_STRIDE(i, n) { r[i] = b[i] - q[i]; }
-}
-__global__ void k_pcg_xr(int n, const double *scalars, double *x, double *r, const double *p, const double *q)
-{
-    double alpha = scalars[S_RZ] / scalars[S_PQ];
-    GRID_STRIDE(i, n)
+    double rr[1] = {0};
+    GRID_STRIDE(i, V.ndof)
     {
-        x[i] += alpha * p[i];
-        r[i] -= alpha * q[i];
+        double v = b[i] - q[i];
+        r[i] = v;
+        rr[0] += v * v;
+    }
+    if (grid_sum<1>(rr, W.part, W.ticket) && threadIdx.x == 0) {
+        V.scalars[S_RR] = rr[0];
+        *W.stop = sqrt(rr[0]) <= tol * sqrt(V.scalars[S_BB]);
     }
 }
-__global__ void k_pcg_p(int n, const double *scalars, double *p, const double *z)
+__global__ void k_pcg_xr(View3 V, double tol, int slot_rz, double *x, double *r, const double *p, const double *q, PcgWork W)
 {
-    double beta = scalars[S_RZNEW] / scalars[S_RZ];
+    if (*W.stop) return;
+    double alpha = V.scalars[slot_rz] / V.scalars[S_PQ];
+    double rr[1] = {0};
+    GRID_STRIDE(i, V.ndof)
+    {
+        x[i] += alpha * p[i];
+        double v = r[i] - alpha * q[i];
+        r[i] = v;
+        rr[0] += v * v;
+    }
+    if (grid_sum<1>(rr, W.part, W.ticket) && threadIdx.x == 0) {
+        V.scalars[S_RR] = rr[0];
+        *W.stop = sqrt(rr[0]) <= tol * sqrt(V.scalars[S_BB]);
+    }
+}
+__global__ void k_pcg_rz(View3 V, int slot, const double *r, const double *z, PcgWork W)
+{
+    if (*W.stop) return;
+    double rz[1] = {0};
+    GRID_STRIDE(i, V.ndof) { rz[0] += r[i] * z[i]; }
+    if (grid_sum<1>(rz, W.part, W.ticket) && threadIdx.x == 0) V.scalars[slot] = rz[0];
+}
+__global__ void k_pcg_p(int n, const double *scalars, int slot_new, int slot_old, double *p, const double *z, const int32_t *stop)
+{
+    if (*stop) return;
+    double beta = scalars[slot_new] / scalars[slot_old];
     GRID_STRIDE(i, n) { p[i] = z[i] + beta * p[i]; }
 }
-__global__ void k_pcg_roll(double *scalars) { scalars[S_RZ] = scalars[S_RZNEW]; }
 }  // namespace ifea

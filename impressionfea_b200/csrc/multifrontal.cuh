@@ -1011,7 +1011,8 @@ public:
                          const double *node_xyz = nullptr) = 0;
     virtual void analyze_from(MfSymbolic &&S) = 0;  // the same, from a symbolic analysis made elsewhere
     virtual void factorize(const double *d_full_vals) = 0;
-    virtual void solve(const double *d_b, double *d_x) = 0;
+    // x = A^-1 b; with `skip`, nothing when *skip (device) is non-zero by the time the sweep starts
+    virtual void solve(const double *d_b, double *d_x, const int32_t *skip) = 0;
     virtual void check_finite(const double *d_x) = 0;
     virtual const MfSymbolic &symbolic() const = 0;
     virtual int64_t factor_nonzeros() const = 0;
@@ -1320,9 +1321,8 @@ public:
             cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, mf::k_sweep<T>, mf::kSwThreads, sweep_smem_), "occupancy");
             // no more CTAs than the widest phase has tiles (and some to wait for the next one)
             sweep_grid_ = std::max(1, std::min(148 * std::max(1, per_sm), width + width / 2));
-            d_cnt_.resize((size_t)mf::kCntN * S.nsuper + 1);
+            d_cnt_.resize((size_t)mf::kCntN * S.nsuper + 2);
             d_cnt_.zero(st_);
-            sweep_epoch_ = 0;
         }
         cuda_check(cudaStreamSynchronize(st_), "cudaStreamSynchronize");
         analyzed_ = true;
@@ -1566,7 +1566,7 @@ public:
     }
 
     // x = A^-1 b on the device (b and x may alias: an entry of x is written after every read of b in its tree).
-    void solve(const double *d_b, double *d_x) override
+    void solve(const double *d_b, double *d_x, const int32_t *skip) override
     {
         if (!factored_) throw Failure(IFEA_BAD_STATE, "Factorize must be called first.");
         const MfSymbolic &S = sym_;
@@ -1576,8 +1576,7 @@ public:
         a.ntasks = (int)d_sweep_.n;
         a.cnt = d_cnt_.p;
         a.ticket = d_cnt_.p + (size_t)mf::kCntN * S.nsuper;
-        a.ticket0 = sweep_epoch_ * (uint32_t)(a.ntasks + sweep_grid_);  // every CTA draws one ticket past the list
-        a.epoch = ++sweep_epoch_;
+        a.skip = profile_ ? nullptr : skip;  // (a profiled solve is a whole one)
         a.perm = d_perm_;
         a.pair = d_pair_.p;
         a.b = d_b;
@@ -1617,7 +1616,6 @@ private:
     {
         d_err_.zero(st_);
         d_cnt_.zero(st_);
-        sweep_epoch_ = 0;
         throw Failure(IFEA_CUDA_ERROR, "multifrontal solve: a wait for another tile timed out");
     }
     void drop_graphs()
@@ -1654,8 +1652,7 @@ private:
     std::vector<int64_t> inv_off_, xinv_off_;
     std::vector<int32_t> small_start_, small_list_, big_start_, big_list_;
     DBuf<mf::SweepTask> d_sweep_;   // the solve's task list
-    DBuf<uint32_t> d_cnt_;          // its completion counters, then the ticket
-    uint32_t sweep_epoch_ = 0;      // solves since the counters were cleared
+    DBuf<uint32_t> d_cnt_;          // its completion counters, then the ticket and the number of solves so far
     int sweep_grid_ = 1;
     std::vector<int> xinv_pass_start_, xinv_task_start_, xinv_pass_kind_;
     DBuf<mf::XTask> d_xinv_tasks_;

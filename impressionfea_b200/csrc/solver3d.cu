@@ -356,7 +356,10 @@ struct Forging3D {
         d_dv, d_er, d_eg, d_ew, d_eenergy, d_epower, d_partials, d_scalars, d_nrm, d_pred, d_nodal, d_q, d_pr, d_pz,
         d_pp, d_pq;
     int vcur = 0;
-    HostPinned<double> hs;
+    HostPinned<double> hs;           // S_COUNT scalars, then those behind an even and an odd PCG iteration
+    cudaEvent_t pcg_ev[2] = {nullptr, nullptr};
+    DBuf<double> d_pcg_part;         // partial sums of a PCG kernel
+    DBuf<int32_t> d_pcg_flag;        // its arrival ticket, the convergence flag
     HostPinned<int32_t> hi;
     int wpb = 8;          // warps per block of the column kernels
     size_t col_smem = 0;  // dynamic shared memory of the column kernels
@@ -371,8 +374,12 @@ struct Forging3D {
         sig_ref = flow_stress(P.C, P.N, P.M, P.eps0, 0, rate_ref);
         k_pen = P.penalty_factor * sig_ref / rate_ref;
         u0 = 5e-3 * P.ram;
-        hs.resize(S_COUNT + 8);
+        hs.resize(3 * S_COUNT);
         hi.resize(8);
+        for (auto &e : pcg_ev) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+        d_pcg_part.resize(4 * kReduceBlocks);
+        d_pcg_flag.resize(2);
+        d_pcg_flag.zero(st);
         d_partials.resize((size_t)S_COUNT * kReduceBlocks);
         d_scalars.resize(S_COUNT);
         d_err.resize(4);
@@ -385,6 +392,8 @@ struct Forging3D {
         join_analysis();
         if (st) cudaStreamSynchronize(st);
         lin.reset();
+        for (auto &e : pcg_ev)
+            if (e) cudaEventDestroy(e);
         if (st && own_stream) cudaStreamDestroy(st);
     }
 
@@ -916,42 +925,57 @@ struct Forging3D {
     {
         View3 V = view();
         int n = topo.ndof;
-        double bb = dot_read(b, b, S_BB);
-        double bnorm = sqrt(bb);
-        if (bnorm == 0) {
-            cuda_check(cudaMemsetAsync(x, 0, n * sizeof(double), st), "memset");
-            return 0;
-        }
         int sp_grid = std::min(kReduceBlocks * 4, (topo.nn * 32 + 255) / 256);
-        lin->solve(b, x);
-        k_spmv<<<sp_grid, 256, 0, st>>>(V, x, d_pq);
-        k_pcg_residual<<<grid(n), 256, 0, st>>>(n, b, d_pq, d_pr);
-        lin->solve(d_pr, d_pz);
+        const PcgWork none = {nullptr, nullptr, nullptr}, W = {d_pcg_part.p, d_pcg_flag.p, d_pcg_flag.p + 1};
+        const int rz[2] = {S_RZ, S_RZNEW};  // r.z of the even and odd iterations
+        // the residual (and |b|^2) of iteration k, copied out behind it; read one iteration later
+        auto post = [&](int k) {
+            cuda_check(cudaMemcpyAsync(hs.p + (1 + (k & 1)) * S_COUNT, d_scalars.p, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H scalars");
+            cuda_check(cudaEventRecord(pcg_ev[k & 1], st), "cudaEventRecord");
+        };
+        auto solve_z = [&](int slot) {
+            lin->solve(d_pr, d_pz, W.stop);
+            k_pcg_rz<<<kReduceBlocks, 256, 0, st>>>(V, slot, d_pr, d_pz, W);
+        };
+        k_dot2<<<kReduceBlocks, 256, 0, st>>>(V, b, b, S_BB, nullptr, 0);
+        finalize({S_BB});
+        lin->solve(b, x, nullptr);
+        k_spmv<<<sp_grid, 256, 0, st>>>(V, x, d_pq, none);
+        k_pcg_residual<<<kReduceBlocks, 256, 0, st>>>(V, tol, b, d_pq, d_pr, W);
+        post(0);
+        solve_z(rz[0]);
         cuda_check(cudaMemcpyAsync(d_pp.p, d_pz.p, n * sizeof(double), cudaMemcpyDeviceToDevice, st), "D2D");
-        k_dot2<<<kReduceBlocks, 256, 0, st>>>(V, d_pr, d_pz, S_RZ, d_pr, S_RR);
-        finalize({S_RZ, S_RR});
-        double rr = read_scalars()[S_RR];
-        double r0 = sqrt(rr);
-        for (int it = 0; it < max_it; it++) {
-            if (sqrt(rr) <= tol * bnorm) return it;
+        double r0 = 0, bnorm = 0;
+        for (int it = 0;; it++) {
+            if (it < max_it) {  // iteration `it`, before its starting residual is known here (the device knows it)
+                k_spmv<<<sp_grid, 256, 0, st>>>(V, d_pp, d_pq, W);
+                k_pcg_xr<<<kReduceBlocks, 256, 0, st>>>(V, tol, rz[it & 1], x, d_pr, d_pp, d_pq, W);
+                post(it + 1);
+                solve_z(rz[(it + 1) & 1]);
+                k_pcg_p<<<grid(n), 256, 0, st>>>(n, d_scalars, rz[(it + 1) & 1], rz[it & 1], d_pp, d_pz, W.stop);
+            }
+            cuda_check(cudaEventSynchronize(pcg_ev[it & 1]), "cudaEventSynchronize");
+            const double *h = hs.p + (1 + (it & 1)) * S_COUNT;
+            const double rr = h[S_RR];
+            if (it == 0) {
+                r0 = sqrt(rr);
+                bnorm = sqrt(h[S_BB]);
+                if (bnorm == 0) {
+                    cuda_check(cudaMemsetAsync(x, 0, n * sizeof(double), st), "memset");
+                    return 0;
+                }
+            } else {
+                lin_its++;
+            }
+            const bool converged = sqrt(rr) <= tol * bnorm;
+            if (it >= max_it) return converged ? max_it : -1;
+            if (converged) return it;
             if (pcg_early_abort && it >= 3) {
                 // the observed contraction cannot reach the tolerance within the budget: refactorise now
                 double rate = pow(sqrt(rr) / r0, 1.0 / it);
                 if (!(rate < 1) || it + log(tol * bnorm / sqrt(rr)) / log(rate) > max_it) return -1;
             }
-            k_spmv<<<sp_grid, 256, 0, st>>>(V, d_pp, d_pq);
-            k_dot2<<<kReduceBlocks, 256, 0, st>>>(V, d_pp, d_pq, S_PQ, nullptr, 0);
-            finalize({S_PQ});
-            k_pcg_xr<<<grid(n), 256, 0, st>>>(n, d_scalars, x, d_pr, d_pp, d_pq);
-            lin->solve(d_pr, d_pz);
-            k_dot2<<<kReduceBlocks, 256, 0, st>>>(V, d_pr, d_pz, S_RZNEW, d_pr, S_RR);
-            finalize({S_RZNEW, S_RR});
-            k_pcg_p<<<grid(n), 256, 0, st>>>(n, d_scalars, d_pp, d_pz);
-            k_pcg_roll<<<1, 1, 0, st>>>(d_scalars);
-            rr = read_scalars()[S_RR];
-            lin_its++;
         }
-        return sqrt(rr) <= tol * bnorm ? max_it : -1;
     }
 
     // PCG iterations a reused factor may take. The reference's budget (PcgBudget, 15) in the FP64 form; in the
@@ -1009,7 +1033,7 @@ struct Forging3D {
                 lin->factorize(d_val);
             }
             if (lin->value_bytes() == 8) {
-                lin->solve(b, x);
+                lin->solve(b, x, nullptr);
                 lin->check_finite(x);
             }
         } catch (Failure &f) {
@@ -1195,7 +1219,7 @@ struct Forging3D {
         cuda_check(cudaEventCreate(&b), "cudaEventCreate");
         cuda_check(cudaEventRecord(a, st), "cudaEventRecord");
         lin->factorize(d_val);
-        lin->solve(d_r, d_dv);
+        lin->solve(d_r, d_dv, nullptr);
         cuda_check(cudaEventRecord(b, st), "cudaEventRecord");
         cuda_check(cudaEventSynchronize(b), "cudaEventSynchronize");
         float ms = 0;

@@ -101,7 +101,7 @@ ifea_status ifea_spd_solve(ifea_spd *h, const double *b, double *x)
     if (!b || !x) return IFEA_INPUT_INVALID;
     return spd_guard(h, [&](ifea_spd &s) {
         s.b.upload(b, s.n, s.st);
-        s.s->solve(s.b, s.x);
+        s.s->solve(s.b, s.x, nullptr);
         s.s->check_finite(s.x);
         s.x.download(x, s.n, s.st);
         ifea::cuda_check(cudaStreamSynchronize(s.st), "cudaStreamSynchronize");

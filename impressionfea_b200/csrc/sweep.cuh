@@ -125,9 +125,8 @@ struct SweepArgs {
     const SweepTask *tasks;
     int ntasks;
     uint32_t *cnt;      // kCntN per front
-    uint32_t *ticket;
-    uint32_t ticket0;   // the ticket counter's value before this solve
-    uint32_t epoch;     // 1 for the first solve after the counters were cleared
+    uint32_t *ticket;   // the next task, zero between solves; then the solves since the counters were cleared
+    const int32_t *skip;  // nothing to do when *skip (null: never)
     const int32_t *perm;
     const int2 *pair;   // per front row: the children's update entries that land on it (see sweep_pairs)
     const double *b;
@@ -520,11 +519,13 @@ static __global__ void __launch_bounds__(kSwThreads, kSwCtas) k_sweep(const Swee
     __shared__ int go[2];  // the task's inputs are complete; 0: a wait gave up
     __shared__ T sa[kSwCompute], yb[PW];
     const int tid = threadIdx.x, lane = tid & 31;
+    if (A.skip && *A.skip) return;
     if (tid >= kSwCompute) {
+        const uint32_t solves = *(volatile uint32_t *)(A.ticket + 1) + 1;
         for (uint32_t i = 0;; i++) {
             const int p = i & 1;
             uint32_t tk = 0;
-            if (lane == 0) tk = atomicAdd(A.ticket, 1u) - A.ticket0;
+            if (lane == 0) tk = atomicAdd(A.ticket, 1u);
             tk = __shfl_sync(0xffffffffu, tk, 0);
             if (i >= 2) sweep_sync(kBarFree + p);  // the computing warps are done with this slot
             const bool have = tk < (uint32_t)A.ntasks;
@@ -533,12 +534,19 @@ static __global__ void __launch_bounds__(kSwThreads, kSwCtas) k_sweep(const Swee
             if (lane == 0 && !have) desc[p].kind = kSwEnd;
             __syncwarp();
             sweep_arrive(kBarDesc + p);
-            if (!have) return;
+            if (!have) {
+                // every CTA draws one ticket past the list: the last of them leaves the counters to the next solve
+                if (lane == 0 && tk == (uint32_t)A.ntasks + gridDim.x - 1) {
+                    A.ticket[0] = 0;
+                    A.ticket[1] = solves;
+                }
+                return;
+            }
             sweep_prefetch(A.D, desc[p], lane);
             int ok = 1;
             if (lane == 0) {
                 const int w = desc[p].wait;
-                ok = w < 0 || sweep_poll(A.cnt + w, A.epoch * (uint32_t)desc[p].target, A.err);
+                ok = w < 0 || sweep_poll(A.cnt + w, solves * (uint32_t)desc[p].target, A.err);
                 if (!ok) atomicExch(A.err, 1);
                 go[p] = ok;
             }
@@ -574,6 +582,10 @@ inline void sweep_pairs(const std::vector<int32_t> &gst, std::vector<int32_t> &s
 {
     const size_t rows = gst.size() - 1;
     pair.resize(std::max<size_t>(rows, 1));
+    size_t more = 0;
+    for (size_t k = 0; k < rows; k++)
+        if (gst[k + 1] - gst[k] > 2) more += gst[k + 1] - gst[k];
+    src.reserve(src.size() + more);
     for (size_t k = 0; k < rows; k++) {
         const int32_t a = gst[k], n = gst[k + 1] - a;
         int2 q = make_int2(n > 0 ? src[a] : -1, n == 2 ? src[a + 1] : -1);
