@@ -4,8 +4,7 @@
 // Per Newton iteration: one thread per quad computes the element stiffness and residual (2x2 Gauss deviatoric
 // power + 1-point volumetric penalty, nodal (t, n) rotation); band cells and residual entries are then gathered in
 // element order (the reference's serial scatter order); fixed DOFs, friction and the band Cholesky follow. The
-// band Cholesky (band.cuh) runs in one CTA, blocked by panels over a circular window of rows in shared memory;
-// every entry's products are subtracted in the same order as the reference's row-oriented loop, so the factor and
+// band Cholesky (band_tri.cuh, band.cuh) runs in one CTA, blocked by columns over a window in shared memory; every entry's products are subtracted in the same order as the reference's row-oriented loop, so the factor and
 // the solution are bit-identical to SymmetricBandMatrix.Factorize / Solve.
 #include <climits>
 #include <cmath>
