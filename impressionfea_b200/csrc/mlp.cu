@@ -1,23 +1,34 @@
 // mlp.cu — the learned warm start's network on the tensor cores: a per-node MLP 16 -> 128 -> 128 -> 128 -> 3 with
 // GELU, BF16 weights and activations, FP32 accumulation, trained by Adam on FP32 master weights.
 //
-// Every layer product is one kernel, k_gemm: C (128-row tiles) = A B^T with A [M][K] and B [N][K] in BF16
-// (K contiguous), staged by cp.async into shared memory as K-major core matrices without swizzle (8 rows x 16 B,
-// one 16-byte K chunk of all rows after another), two stages deep, multiplied by tcgen05.mma kind::f16 issued by
-// one thread into a tensor-memory accumulator, and read back by tcgen05.ld for a fused epilogue:
-//   forward hidden layer  z = acc + b, h = GELU(z)        (z kept in FP32 for the backward pass, h in BF16 both
-//                                                          [row][feature] and transposed)
-//   backward hidden layer dz = acc * GELU'(z)             (BF16, both layouts)
-//   weight gradient       partial sums over a K slice     (FP32; K = the batch, split over CTAs, summed in order)
-// The 3-wide output layer, the loss and its gradient, the bias gradients and Adam are small SIMT kernels.
-// Every sum runs in a fixed order, so training is bit-reproducible run to run.
+// A training step is three launches:
+//   k_tile    per 128 rows of the batch, one CTA takes them through the whole network: gather and normalise, three hidden
+//             layers, output layer, loss, and back to the first layer's gradient. Activations and layer gradients stay
+//             in shared memory as the next product's operand (K-major core matrices without swizzle: 8 rows x 16 B, one
+//             16-byte K chunk of all rows after another), pre-activations and then GELU' in tensor memory (three
+//             accumulators of 128 columns, a fourth for the backward products); products are tcgen05.mma kind::f16 issued by one
+//             thread. Only what the weight gradients need leaves the CTA: activations and layer gradients, transposed.
+//   k_wgrad   the weight gradients: partial sums over slices of 512 batch rows (FP32, summed in order by k_update), a
+//             slice's operands for 128 x 64 of a gradient all in shared memory, multiplied as they land;
+//   k_update  sums the partial sums, the bias gradients and Adam, and the BF16 copies of the new weights.
+// Inference is k_tile without the backward half, over all rows in one launch. Every sum runs in a fixed order, so
+// training is bit-reproducible run to run.
+//
+// What bounds a step of 8,192 rows (B200): the chain inside k_tile, 27 us of the step's 47 on the device. It starts
+// with 5 us of dependent loads (index, row, normalisation); an epilogue of 128 x 128 GELUs and their derivatives is
+// 6,100 cycles of issue on one SM, 8,000 with the transposed stores, a product with its wait 300 - 800. k_wgrad takes
+// 11.5 us (16 with a ring of four stages over slices of the whole width), k_update 5.6. A step through the public class
+// takes 53 us; with a kernel for each layer and each sum, 21 launches a step with pre-activations, activations and
+// transposes through global memory and a wait for the device in every step, it took 336.
 #include <cuda_bf16.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <future>
 #include <numeric>
 #include <random>
+#include <system_error>
 
 #include "warmstart.h"
 
@@ -25,6 +36,7 @@ namespace ifea {
 namespace wsm {
 
 constexpr int BM = 128, BK = 64, SPLIT_K = 512;
+constexpr int kTileThreads = 512, kGradN = 64, kGradStages = SPLIT_K / BK;
 typedef __nv_bfloat16 bf16;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -69,6 +81,28 @@ __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, int by
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
 
+// until at most `left` of this thread's groups of copies are in flight (left is known at compile time: one case stays)
+__device__ __forceinline__ void cp_async_wait(int left)
+{
+    switch (left) {
+    case 7: asm volatile("cp.async.wait_group 7;" ::: "memory"); break;
+    case 6: asm volatile("cp.async.wait_group 6;" ::: "memory"); break;
+    case 5: asm volatile("cp.async.wait_group 5;" ::: "memory"); break;
+    case 4: asm volatile("cp.async.wait_group 4;" ::: "memory"); break;
+    case 3: asm volatile("cp.async.wait_group 3;" ::: "memory"); break;
+    case 2: asm volatile("cp.async.wait_group 2;" ::: "memory"); break;
+    case 1: asm volatile("cp.async.wait_group 1;" ::: "memory"); break;
+    default: asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+}
+
+#define WSM_TMEM_ST16(taddr, r)                                                                                      \
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], "                                                     \
+                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"((r)[0]), "r"((r)[1]), "r"((r)[2]),   \
+                 "r"((r)[3]), "r"((r)[4]), "r"((r)[5]), "r"((r)[6]), "r"((r)[7]), "r"((r)[8]), "r"((r)[9]),            \
+                 "r"((r)[10]), "r"((r)[11]), "r"((r)[12]), "r"((r)[13]), "r"((r)[14]), "r"((r)[15]), "r"(taddr)        \
+                 : "memory")
+
 #define WSM_TMEM_LD16(taddr, r)                                                                                      \
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "  \
                  "[%16];"                                                                                            \
@@ -83,298 +117,472 @@ __device__ __forceinline__ float gelu_d(float z)
     return 0.5f * (1.0f + erff(z * 0.70710678118654752f)) + z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
-enum { EPI_FWD = 0, EPI_BWD = 1, EPI_PART = 2 };
+constexpr uint32_t kChunk = BM * 16;             // one 8-column chunk of 128 rows in shared memory
+constexpr int kMat = BM * HID * 2;                // a 128 x 128 operand, 32 KB
+// element (r, k) of an operand of 128 rows
+__host__ __device__ constexpr int core(int r, int k) { return ((k >> 3) * BM + r) * 8 + (k & 7); }
 
-struct Gemm {
-    const bf16 *A;
-    int64_t lda;  // [M][K]
-    const bf16 *B;
-    int64_t ldb;  // [N][K]
-    int M, K, kper;
-    const float *bias;  // EPI_FWD
-    const float *zin;   // EPI_BWD: pre-activations [M][N]
-    float *zout;        // EPI_FWD: pre-activations out [M][N] (or null)
-    bf16 *h;            // [M][N] (row stride N)
-    bf16 *ht;           // [N][M] (row stride ldht) or null
-    int64_t ldht;
-    float *part;  // EPI_PART: [split][M][N]
+struct Tile {
+    const float *x, *t;      // raw inputs [.][16] and targets [.][3]
+    const int32_t *idx;      // the rows of the batch (null: 0, 1, ..)
+    int64_t n;               // rows of x
+    int M;                   // rows of the batch (training: a multiple of 128)
+    const float *norm, *par;
+    const bf16 *w1, *w2, *w3, *w2t, *w3t;  // weights as operands
+    float *y;                // inference: raw outputs [M][3]
+    bf16 *xbt, *h1t, *h2t, *dz1t, *dz2t, *dz3t;  // training: [feature][M]
+    float *hpart;            // per tile: dW4, db4, the loss
     int *err;
 };
 
-template <int N>
-constexpr int gemm_smem() { return 2 * (BM * BK * 2) + 2 * (N * BK * 2) + 64; }
+// shared memory: weights, activations, (training) transposed weights and layer gradient; inputs, W1; small vectors
+template <bool TRAIN>
+constexpr int tile_smem() { return (TRAIN ? 6 : 3) * kMat + 2 * BM * NIN * 2 + (3 * HID + NOUT * HID + NOUT + 1) * 4 + 128 * 4 * 4 + 64; }
 
-template <int N, int EPI>
-__global__ void __launch_bounds__(128) k_gemm(Gemm g)
+template <bool TRAIN>
+__global__ void __launch_bounds__(kTileThreads, 1) k_tile(Tile g)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
-    constexpr int A_STAGE = BM * BK * 2, B_STAGE = N * BK * 2;
-    constexpr uint32_t CHUNK_A = BM * 16, CHUNK_B = N * 16;
-    constexpr int TCOLS = N < 32 ? 32 : N;
-    uint64_t *bar = (uint64_t *)(sm + 2 * A_STAGE + 2 * B_STAGE);
-    uint32_t *tslot = (uint32_t *)(bar + 2);
+    constexpr int TCOLS = TRAIN ? 512 : 128;
+    bf16 *sw2 = (bf16 *)sm, *sw3 = sw2 + kMat / 2, *sh = sw3 + kMat / 2;  // sh: the activations
+    bf16 *sw2t = sh + kMat / 2, *sw3t = sw2t + kMat / 2, *sdz = sw3t + kMat / 2;
+    bf16 *sx = TRAIN ? sdz + kMat / 2 : sw2t, *sw1 = sx + BM * NIN;
+    float *sbias = (float *)(sw1 + BM * NIN), *sw4 = sbias + 3 * HID;  // b1, b2, b3; W4, b4
+    float *dys = sw4 + NOUT * HID + NOUT + 1, *red = dys + 128 * NOUT;
+    uint64_t *bar = (uint64_t *)(((uintptr_t)(red + 128) + 15) & ~(uintptr_t)15);
+    uint32_t *tslot = (uint32_t *)(bar + 1);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * BM, split = blockIdx.y;
-    const int k0 = split * g.kper, k1 = min(g.K, k0 + g.kper);
-    const uint32_t sbase = smem_u32(sm);
+    const int m0 = blockIdx.x * BM;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(TCOLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
     if (tid == 0) {
-        for (int s = 0; s < 2; s++) asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar + s)), "r"(1));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(1));
         asm volatile("fence.mbarrier_init.release.cluster;" ::);
     }
+    // weights (already in operand form) asynchronously, behind the first layer
+    auto load = [&](bf16 *dst, const bf16 *src, int bytes) {
+        for (int q = tid; q < bytes / 16; q += kTileThreads) cp_async16(smem_u32(dst) + 16 * q, (const uint4 *)src + q, 16);
+    };
+    load(sw1, g.w1, BM * NIN * 2);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    load(sw2, g.w2, kMat);
+    load(sw3, g.w3, kMat);
+    if (TRAIN) {
+        load(sw2t, g.w2t, kMat);
+        load(sw3t, g.w3t, kMat);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    for (int i = tid; i < HID; i += kTileThreads) {
+        sbias[i] = g.par[OFF_B1 + i];
+        sbias[HID + i] = g.par[OFF_B2 + i];
+        sbias[2 * HID + i] = g.par[OFF_B3 + i];
+    }
+    for (int i = tid; i < NOUT * HID + NOUT; i += kTileThreads) sw4[i] = g.par[OFF_W4 + i];
+    // normalised inputs, four columns a thread; rows past the data are zero. Threads 0 .. 127 keep their row's targets
+    float tgt[NOUT];
+    {
+        const int r = tid & 127, c0 = 4 * (tid >> 7), row = m0 + r;
+        int64_t src = row < g.M ? (int64_t)row : g.n;
+        if (TRAIN && g.idx) {  // (host memory: each index is read once)
+            if (tid < BM) ((int32_t *)dys)[tid] = g.idx[row];
+            __syncthreads();
+            src = ((int32_t *)dys)[r];
+        }
+        float v[4] = {0, 0, 0, 0};
+        if (src < g.n) {
+            const float4 q = *(const float4 *)(g.x + src * NIN + c0);
+            v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+#pragma unroll
+            for (int j = 0; j < 4; j++) v[j] = (v[j] - g.norm[c0 + j]) / g.norm[NIN + c0 + j];
+        }
+        __align__(8) bf16 hb[4];
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            hb[j] = __float2bfloat16_rn(v[j]);
+            if (TRAIN) g.xbt[(int64_t)(c0 + j) * g.M + row] = hb[j];
+        }
+        *(uint2 *)(sx + core(r, c0)) = *(const uint2 *)hb;
+        if (TRAIN && tid < BM)
+#pragma unroll
+            for (int o = 0; o < NOUT; o++)
+                tgt[o] = src < g.n ? (g.t[src * NOUT + o] - g.norm[2 * NIN + o]) / g.norm[2 * NIN + NOUT + o] : 0.0f;
+    }
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::);
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::);
     const uint32_t tmem = *tslot;
-    const int nblk = (k1 - k0 + BK - 1) / BK;
-    uint32_t ph[2] = {0, 0};
+    uint32_t phase = 0;
     bool ok = true;
-    for (int b = 0; b < nblk; b++) {
-        const int s = b & 1;
-        if (b >= 2) {
-            ok = mbar_wait(smem_u32(bar + s), ph[s]);
-            ph[s] ^= 1;
-            if (__syncthreads_or(!ok)) break;
+    // D(columns col ..) = A B^T over K columns; every thread sees the result when it returns
+    auto product = [&](const bf16 *A, const bf16 *B, int K, uint32_t col) {
+        if (tid == 0) {
+            const uint32_t sa = smem_u32(A), sb = smem_u32(B);
+            for (int j = 0; j < K / 16; j++)
+                mma_bf16(tmem + col, sdesc(sa + j * 2 * kChunk, kChunk), sdesc(sb + j * 2 * kChunk, kChunk), idesc<HID>(), j > 0);
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)));
         }
-        const int kb = k0 + b * BK, kn = min(BK, k1 - kb);
-        const uint32_t sa = sbase + s * A_STAGE, sb = sbase + 2 * A_STAGE + s * B_STAGE;
-        for (int q = tid; q < BM * 8; q += 128) {
-            int r = q >> 3, c = q & 7, row = m0 + r;
-            bool v = row < g.M && 8 * c < kn;
-            const void *src = v ? (const void *)(g.A + (int64_t)row * g.lda + kb + 8 * c) : (const void *)g.A;
-            cp_async16(sa + (uint32_t)(c * BM + r) * 16, src, v ? 16 : 0);
-        }
-        for (int q = tid; q < N * 8; q += 128) {
-            int r = q >> 3, c = q & 7;
-            bool v = 8 * c < kn;
-            const void *src = v ? (const void *)(g.B + (int64_t)r * g.ldb + kb + 8 * c) : (const void *)g.B;
-            cp_async16(sb + (uint32_t)(c * N + r) * 16, src, v ? 16 : 0);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        ok = mbar_wait(smem_u32(bar), phase) && ok;
+        phase ^= 1;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::);
+    };
+    // before a product: this CTA's writes to shared memory and reads of tensor memory are done
+    auto settle = [&]() {
+        asm volatile("tcgen05.fence::before_thread_sync;" ::);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();
-        if (tid == 0) {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::);
-            for (int j = 0; j < kn / 16; j++)
-                mma_bf16(tmem, sdesc(sa + j * 2 * CHUNK_A, CHUNK_A), sdesc(sb + j * 2 * CHUNK_B, CHUNK_B), idesc<N>(),
-                         (b > 0 || j > 0) ? 1u : 0u);
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar + s)));
-        }
-    }
-    if (ok && nblk > 0) {
-        const int s = (nblk - 1) & 1;
-        ok = mbar_wait(smem_u32(bar + s), ph[s]);
-    }
-    if (__syncthreads_or(!ok)) {
-        if (tid == 0) atomicExch(g.err, 1);
-    } else {
         asm volatile("tcgen05.fence::after_thread_sync;" ::);
-        const int r = 32 * warp + lane, row = m0 + r;
+    };
+    // a thread's part of an epilogue: row r, columns cb .. cb + 31. Training leaves GELU'(z) where z was, for the way
+    // back: the two share the error function, which is what an epilogue spends its time on
+    const int r = 32 * (warp & 3) + lane, cb = 32 * (warp >> 2), row = m0 + r;
+    const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)cb;
+    auto hidden = [&](uint32_t col, const float *bias, bf16 *ht) {
 #pragma unroll 1
-        for (int c0 = 0; c0 < N; c0 += 16) {
+        for (int h = 0; h < 2; h++) {
             uint32_t v[16];
-            WSM_TMEM_LD16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)c0, v);
+            WSM_TMEM_LD16(tl + col + 16 * h, v);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (row >= g.M) continue;
-            if (EPI == EPI_PART) {
-                float *dst = g.part + ((int64_t)split * g.M + row) * N + c0;
-#pragma unroll
-                for (int j = 0; j < 16; j++) dst[j] = __uint_as_float(v[j]);
-                continue;
-            }
-            float o[16];
-#pragma unroll
-            for (int j = 0; j < 16; j++) {
-                float a = __uint_as_float(v[j]);
-                if (EPI == EPI_FWD) {
-                    float z = a + g.bias[c0 + j];
-                    if (g.zout) g.zout[(int64_t)row * N + c0 + j] = z;
-                    o[j] = gelu(z);
-                } else {
-                    o[j] = a * gelu_d(g.zin[(int64_t)row * N + c0 + j]);
-                }
-            }
             __align__(16) bf16 hb[16];
 #pragma unroll
-            for (int j = 0; j < 16; j++) hb[j] = __float2bfloat16_rn(o[j]);
-            uint4 *dst = (uint4 *)(g.h + (int64_t)row * N + c0);
-            dst[0] = ((const uint4 *)hb)[0];
-            dst[1] = ((const uint4 *)hb)[1];
-            if (g.ht)
+            for (int j = 0; j < 16; j++) {
+                const float z = __uint_as_float(v[j]) + bias[cb + 16 * h + j];
+                hb[j] = __float2bfloat16_rn(gelu(z));
+                if (TRAIN) v[j] = __float_as_uint(gelu_d(z));
+            }
+            if (TRAIN) WSM_TMEM_ST16(tl + col + 16 * h, v);
+            *(uint4 *)(sh + core(r, cb + 16 * h)) = ((const uint4 *)hb)[0];
+            *(uint4 *)(sh + core(r, cb + 16 * h + 8)) = ((const uint4 *)hb)[1];
+            if (TRAIN && ht)
 #pragma unroll
-                for (int j = 0; j < 16; j++) g.ht[(int64_t)(c0 + j) * g.ldht + row] = hb[j];
+                for (int j = 0; j < 16; j++) ht[(int64_t)(cb + 16 * h + j) * g.M + row] = hb[j];
+        }
+        if (TRAIN) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    };
+    product(sx, sw1, NIN, 0);
+    hidden(0, sbias, g.h1t);
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    settle();
+    product(sh, sw2, HID, TRAIN ? HID : 0);
+    hidden(TRAIN ? HID : 0, sbias + HID, g.h2t);
+    settle();
+    product(sh, sw3, HID, TRAIN ? 2 * HID : 0);
+    hidden(TRAIN ? 2 * HID : 0, sbias + 2 * HID, nullptr);
+    __syncthreads();
+    // output layer (FP32 over the BF16 activations), a row a thread
+    if (tid < BM) {
+        float acc[NOUT];
+#pragma unroll
+        for (int o = 0; o < NOUT; o++) acc[o] = sw4[NOUT * HID + o];
+#pragma unroll 4
+        for (int q = 0; q < HID / 8; q++) {
+            const uint4 u = *(const uint4 *)(sh + core(tid, 8 * q));
+            const bf16 *hv = (const bf16 *)&u;
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float hf = __bfloat162float(hv[j]);
+#pragma unroll
+                for (int o = 0; o < NOUT; o++) acc[o] += sw4[o * HID + 8 * q + j] * hf;
+            }
+        }
+        const int mr = m0 + tid;
+        if (!TRAIN) {
+            if (mr < g.M)
+                for (int o = 0; o < NOUT; o++) g.y[(int64_t)mr * NOUT + o] = g.norm[2 * NIN + o] + g.norm[2 * NIN + NOUT + o] * acc[o];
+        } else {
+            // the loss and its gradient at the output
+            const float scale = 2.0f / (float)(g.M * NOUT);
+            float l = 0;
+#pragma unroll
+            for (int o = 0; o < NOUT; o++) {
+                const float e = acc[o] - tgt[o];
+                l += e * e;
+                dys[tid * NOUT + o] = scale * e;
+            }
+            red[tid] = l;
+        }
+    }
+    if (TRAIN) {
+        __syncthreads();
+        // dz3 = (dy W4) * GELU'(z3)
+        float dy[NOUT];
+#pragma unroll
+        for (int o = 0; o < NOUT; o++) dy[o] = dys[r * NOUT + o];
+#pragma unroll 1
+        for (int h = 0; h < 2; h++) {
+            uint32_t v[16];
+            WSM_TMEM_LD16(tl + 2 * HID + 16 * h, v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            __align__(16) bf16 hb[16];
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const int i = cb + 16 * h + j;
+                float dh = 0;
+#pragma unroll
+                for (int o = 0; o < NOUT; o++) dh += dy[o] * sw4[o * HID + i];
+                hb[j] = __float2bfloat16_rn(dh * __uint_as_float(v[j]));
+                g.dz3t[(int64_t)i * g.M + row] = hb[j];
+            }
+            *(uint4 *)(sdz + core(r, cb + 16 * h)) = ((const uint4 *)hb)[0];
+            *(uint4 *)(sdz + core(r, cb + 16 * h + 8)) = ((const uint4 *)hb)[1];
+        }
+        settle();
+        if (warp >= 12) {
+            // dW4[o][i] = sum over the tile's rows of dy[o] h3[row][i]: a thread owns column i; then db4
+            float *out = g.hpart + (int64_t)blockIdx.x * (NOUT * HID + NOUT + 1);
+            const int i = tid - 384;
+            float acc[NOUT] = {0, 0, 0};
+#pragma unroll 8
+            for (int k = 0; k < BM; k++) {
+                const float hv = __bfloat162float(sh[core(k, i)]);
+#pragma unroll
+                for (int o = 0; o < NOUT; o++) acc[o] += dys[k * NOUT + o] * hv;
+            }
+            for (int o = 0; o < NOUT; o++) out[o * HID + i] = acc[o];
+            if (i < NOUT) {
+                float s = 0;
+                for (int k = 0; k < BM; k++) s += dys[k * NOUT + i];
+                out[NOUT * HID + i] = s;
+            }
+        } else if (warp == 11) {
+            // the loss: the 128 rows' squares by a tree of halves (64, 32, .. apart)
+            float q[4];
+            for (int k = 0; k < 4; k++) q[k] = red[lane + 32 * k];
+            float s = (q[0] + q[2]) + (q[1] + q[3]);
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+            if (lane == 0) g.hpart[(int64_t)blockIdx.x * (NOUT * HID + NOUT + 1) + NOUT * HID + NOUT] = s;
+        }
+        // back through the hidden layers: dz = (dz above W) * GELU'(z)
+        auto back = [&](uint32_t zcol, bf16 *dzt, bool keep) {
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) {
+                uint32_t v[16], z[16];
+                WSM_TMEM_LD16(tl + 3 * HID + 16 * h, v);
+                WSM_TMEM_LD16(tl + zcol + 16 * h, z);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                __align__(16) bf16 hb[16];
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const int i = cb + 16 * h + j;
+                    hb[j] = __float2bfloat16_rn(__uint_as_float(v[j]) * __uint_as_float(z[j]));
+                    dzt[(int64_t)i * g.M + row] = hb[j];
+                }
+                if (keep) {
+                    *(uint4 *)(sdz + core(r, cb + 16 * h)) = ((const uint4 *)hb)[0];
+                    *(uint4 *)(sdz + core(r, cb + 16 * h + 8)) = ((const uint4 *)hb)[1];
+                }
+            }
+        };
+        product(sdz, sw3t, HID, 3 * HID);
+        back(HID, g.dz2t, true);
+        settle();
+        product(sdz, sw2t, HID, 3 * HID);
+        back(0, g.dz1t, false);
+    }
+    if (__syncthreads_or(!ok) && tid == 0) atomicExch(g.err, 1);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::);
+    __syncthreads();
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS));
+}
+
+// Partial weight gradients: part[split][layer] = dz^T h over a slice of 512 batch rows (operands [feature][batch], K-major).
+struct Grad {
+    const bf16 *A[3], *B[3];  // dz3^T h2^T, dz2^T h1^T, dz1^T x^T
+    float *part[3];           // [split][128][128], the last [split][128][16]
+    int M;                    // the batch
+    int *err;
+};
+constexpr int grad_smem() { return kGradStages * (BM + kGradN) * BK * 2 + 64; }
+
+// columns n0 .. n0 + N - 1 of slice `split` of a gradient [128][ldp]
+template <int N>
+__device__ __forceinline__ void grad_slice(const bf16 *A, const bf16 *B, int ld, float *part, int ldp, int n0, int split, int *err)
+{
+    extern __shared__ __align__(1024) unsigned char sm[];
+    constexpr int A_BYTES = BM * BK * 2, STAGE = A_BYTES + kGradN * BK * 2;
+    constexpr uint32_t CHUNK_B = N * 16;
+    constexpr int TCOLS = N < 32 ? 32 : N;
+    uint64_t *bar = (uint64_t *)(sm + kGradStages * STAGE);
+    uint32_t *tslot = (uint32_t *)(bar + 1);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int k0 = split * SPLIT_K, nblk = (min(ld, k0 + SPLIT_K) - k0) / BK;  // (ld: a multiple of 128)
+    const uint32_t sbase = smem_u32(sm);
+    for (int b = 0; b < kGradStages; b++) {  // 64 batch rows a stage: 8 chunks of 8, lanes over 16 features x 2 chunks
+        if (b < nblk) {
+            const int kb = k0 + b * BK;
+            const uint32_t sa = sbase + b * STAGE, sb = sa + A_BYTES;
+            for (int q = tid; q < BM * 8; q += 256) {
+                const int c = 2 * (q / (2 * BM)) + (q & 1), r = (q >> 1) % BM;
+                cp_async16(sa + (uint32_t)(c * BM + r) * 16, A + (int64_t)r * ld + kb + 8 * c, 16);
+            }
+            for (int q = tid; q < N * 8; q += 256) {
+                const int c = 2 * (q / (2 * N)) + (q & 1), r = (q >> 1) % N;
+                cp_async16(sb + (uint32_t)(c * N + r) * 16, B + (int64_t)(n0 + r) * ld + kb + 8 * c, 16);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)), "r"(TCOLS));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(1));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::);
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::);
+    const uint32_t tmem = *tslot;
+#pragma unroll
+    for (int b = 0; b < kGradStages; b++) {
+        cp_async_wait(kGradStages - 1 - b);  // block b has landed
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        if (tid == 0 && b < nblk) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::);
+            const uint32_t sa = sbase + b * STAGE, sb = sa + A_BYTES;
+            for (int j = 0; j < BK / 16; j++)
+                mma_bf16(tmem, sdesc(sa + j * 2 * kChunk, kChunk), sdesc(sb + j * 2 * CHUNK_B, CHUNK_B), idesc<N>(), (b > 0 || j > 0) ? 1u : 0u);
+        }
+    }
+    if (tid == 0) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)));
+    const bool ok = mbar_wait(smem_u32(bar), 0);
+    if (__syncthreads_or(!ok)) {
+        if (tid == 0) atomicExch(err, 1);
+    } else {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::);
+        const int r = 32 * (warp & 3) + lane;
+#pragma unroll 1
+        for (int c0 = 16 * (warp >> 2); c0 < N; c0 += 32) {
+            uint32_t v[16];
+            WSM_TMEM_LD16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)c0, v);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            float4 *dst = (float4 *)(part + ((int64_t)split * BM + r) * ldp + n0 + c0);
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+                dst[j] = make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3]));
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::);
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TCOLS));
 }
-
-// ------------------------------------------------------------------ SIMT parts
-
-// rows of normalised inputs in BF16, [M][16] and transposed [16][ldt]; rows past n are zero
-__global__ void k_pack_inputs(const float *__restrict__ x, const int32_t *__restrict__ idx, int64_t n, int M,
-                              const float *__restrict__ norm, bf16 *__restrict__ xb, bf16 *__restrict__ xbt, int ldt,
-                              const float *__restrict__ t, float *__restrict__ tb)
+__global__ void __launch_bounds__(256) k_wgrad(Grad g)
 {
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < M; r += gridDim.x * blockDim.x) {
-        int64_t src = idx ? (int64_t)idx[r] : (int64_t)r;
-        bool v = src < n;
-        __align__(16) bf16 hb[NIN];
-        for (int c = 0; c < NIN; c++) {
-            float a = v ? (x[src * NIN + c] - norm[c]) / norm[NIN + c] : 0.0f;
-            hb[c] = __float2bfloat16_rn(a);
-            if (xbt) xbt[(int64_t)c * ldt + r] = hb[c];
-        }
-        uint4 *d = (uint4 *)(xb + (int64_t)r * NIN);
-        d[0] = ((const uint4 *)hb)[0];
-        d[1] = ((const uint4 *)hb)[1];
-        if (tb)
-            for (int o = 0; o < NOUT; o++)
-                tb[(int64_t)r * NOUT + o] = v ? (t[src * NOUT + o] - norm[2 * NIN + o]) / norm[2 * NIN + NOUT + o] : 0.0f;
+    constexpr int PER = HID / kGradN;
+    if (blockIdx.y < 2 * PER) {
+        const int n0 = kGradN * (blockIdx.y % PER);
+        if (blockIdx.y < PER) grad_slice<kGradN>(g.A[0], g.B[0], g.M, g.part[0], HID, n0, blockIdx.x, g.err);
+        else grad_slice<kGradN>(g.A[1], g.B[1], g.M, g.part[1], HID, n0, blockIdx.x, g.err);
+    } else {
+        grad_slice<NIN>(g.A[2], g.B[2], g.M, g.part[2], NIN, 0, blockIdx.x, g.err);
     }
 }
 
-// output layer y = W4 h3 + b4 (FP32 over the BF16 activations); denorm != 0 maps back to raw targets
-__global__ void k_head_fwd(const bf16 *__restrict__ h3, int M, const float *__restrict__ par, const float *__restrict__ norm,
-                           int denorm, float *__restrict__ y)
-{
-    __shared__ float w[NOUT * HID + NOUT];
-    for (int i = threadIdx.x; i < NOUT * HID + NOUT; i += blockDim.x) w[i] = par[OFF_W4 + i];
-    __syncthreads();
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < M; r += gridDim.x * blockDim.x) {
-        float acc[NOUT];
-        for (int o = 0; o < NOUT; o++) acc[o] = w[NOUT * HID + o];
-        const uint4 *row = (const uint4 *)(h3 + (int64_t)r * HID);
-        for (int q = 0; q < HID / 8; q++) {
-            uint4 u = row[q];
-            const bf16 *hv = (const bf16 *)&u;
-            for (int j = 0; j < 8; j++) {
-                float hf = __bfloat162float(hv[j]);
-                for (int o = 0; o < NOUT; o++) acc[o] += w[o * HID + 8 * q + j] * hf;
-            }
-        }
-        for (int o = 0; o < NOUT; o++)
-            y[(int64_t)r * NOUT + o] = denorm ? norm[2 * NIN + o] + norm[2 * NIN + NOUT + o] * acc[o] : acc[o];
-    }
-}
-
-// loss and its gradient at the output, back through the output layer: dz3 = (dy W4) * GELU'(z3); per-block
-// partial sums of dW4, db4 and the loss (rows past n contribute nothing)
-__global__ void __launch_bounds__(128) k_head_bwd(const bf16 *__restrict__ h3, const float *__restrict__ z3,
-                                                  const float *__restrict__ y, const float *__restrict__ t, int n, int M,
-                                                  const float *__restrict__ par, bf16 *__restrict__ dz3,
-                                                  bf16 *__restrict__ dz3t, float *__restrict__ hpart)
-{
-    __shared__ float w[NOUT * HID];
-    __shared__ float dys[128][NOUT];
-    __shared__ float red[128];
-    for (int i = threadIdx.x; i < NOUT * HID; i += blockDim.x) w[i] = par[OFF_W4 + i];
-    int r = blockIdx.x * 128 + threadIdx.x;
-    float dy[NOUT], l = 0;
-    const float scale = 2.0f / (float)(n * NOUT);
-    for (int o = 0; o < NOUT; o++) {
-        float e = r < n ? y[(int64_t)r * NOUT + o] - t[(int64_t)r * NOUT + o] : 0.0f;
-        l += e * e;
-        dy[o] = scale * e;
-        dys[threadIdx.x][o] = dy[o];
-    }
-    __syncthreads();
-    if (r < M) {
-        for (int c0 = 0; c0 < HID; c0 += 8) {
-            __align__(16) bf16 hb[8];
-            for (int j = 0; j < 8; j++) {
-                int i = c0 + j;
-                float dh = 0;
-                for (int o = 0; o < NOUT; o++) dh += dy[o] * w[o * HID + i];
-                hb[j] = __float2bfloat16_rn(dh * gelu_d(z3[(int64_t)r * HID + i]));
-                dz3t[(int64_t)i * M + r] = hb[j];
-            }
-            *(uint4 *)(dz3 + (int64_t)r * HID + c0) = *(const uint4 *)hb;
-        }
-    }
-    // dW4[o][i] = sum over this block's rows of dy[o] h3[row][i]: thread i owns column i
-    float* out = hpart + (int64_t)blockIdx.x * (NOUT * HID + NOUT + 1);
+// BF16 copies of a hidden weight as operands: W by rows of outputs for the forward products, W^T for the backward ones
+struct Weights {
+    bf16 *w1, *w2, *w3, *w2t, *w3t;
+    __device__ __forceinline__ void publish(int p, float v) const
     {
-        int i = threadIdx.x;
-        float acc[NOUT] = {0, 0, 0};
-        for (int k = 0; k < 128; k++) {
-            int rr = blockIdx.x * 128 + k;
-            if (rr >= M) break;
-            float hv = __bfloat162float(h3[(int64_t)rr * HID + i]);
-            for (int o = 0; o < NOUT; o++) acc[o] += dys[k][o] * hv;
+        const bf16 a = __float2bfloat16_rn(v);
+        if (p >= OFF_W1 && p < OFF_W1 + HID * NIN) {
+            w1[core((p - OFF_W1) / NIN, (p - OFF_W1) % NIN)] = a;
+        } else if (p >= OFF_W2 && p < OFF_W2 + HID * HID) {
+            w2[core((p - OFF_W2) / HID, (p - OFF_W2) % HID)] = a;
+            w2t[core((p - OFF_W2) % HID, (p - OFF_W2) / HID)] = a;
+        } else if (p >= OFF_W3 && p < OFF_W3 + HID * HID) {
+            w3[core((p - OFF_W3) / HID, (p - OFF_W3) % HID)] = a;
+            w3t[core((p - OFF_W3) % HID, (p - OFF_W3) / HID)] = a;
         }
-        for (int o = 0; o < NOUT; o++) out[o * HID + i] = acc[o];
     }
-    if (threadIdx.x < NOUT) {
-        float acc = 0;
-        for (int k = 0; k < 128; k++) acc += dys[k][threadIdx.x];
-        out[NOUT * HID + threadIdx.x] = acc;
-    }
-    red[threadIdx.x] = l;
-    __syncthreads();
-    for (int s = 64; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[NOUT * HID + NOUT] = red[0];
+};
+__global__ void k_publish(const float *__restrict__ par, Weights w)
+{
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < NPAR; p += gridDim.x * blockDim.x) w.publish(p, par[p]);
 }
 
-// out[i] = sum over parts j (in order) of p[j * count + i]
-__global__ void k_sum_parts(const float *__restrict__ p, int nparts, int count, int stride, float *__restrict__ out)
+// The gradient of every parameter from the partial sums (in order), and with lr != 0 one Adam step and the new
+// weights' copies. Blocks 0 .. 3 HID - 1: a bias each, its layer gradient's row [HID][M] summed (fixed order); then a
+// weight (or an output bias) a thread; the last thread the batch loss, when wanted.
+struct Update {
+    const bf16 *dzt[3];   // layers 3, 2, 1
+    const float *part[3], *hpart;
+    int M, splits, nblk;
+    float *grad, *par, *m, *v, *loss;
+    float lr, bc1, bc2;
+    Weights w;
+};
+__device__ __forceinline__ void adam(const Update &u, int p, float gi)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        float acc = 0;
-        for (int j = 0; j < nparts; j++) acc += p[(int64_t)j * stride + i];
-        out[i] = acc;
-    }
-}
-
-// bias gradients: row f of the transposed layer gradient [HID][M] summed (block per feature, fixed order)
-__global__ void k_row_sums(const bf16 *__restrict__ dzt, int M, float *__restrict__ out)
-{
-    __shared__ float red[256];
-    const bf16 *row = dzt + (int64_t)blockIdx.x * M;
-    float acc = 0;
-    for (int i = threadIdx.x; i < M; i += blockDim.x) acc += __bfloat162float(row[i]);
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) out[blockIdx.x] = red[0];
-}
-
-__global__ void k_adam(float *__restrict__ w, const float *__restrict__ g, float *__restrict__ m, float *__restrict__ v,
-                       int n, float lr, float bc1, float bc2)
-{
+    u.grad[p] = gi;
+    if (u.lr == 0.0f) return;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float gi = g[i];
-        float mi = b1 * m[i] + (1 - b1) * gi, vi = b2 * v[i] + (1 - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        w[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-    }
+    const float mi = b1 * u.m[p] + (1 - b1) * gi, vi = b2 * u.v[p] + (1 - b2) * gi * gi;
+    u.m[p] = mi;
+    u.v[p] = vi;
+    const float w = u.par[p] - u.lr * (mi / u.bc1) / (sqrtf(vi / u.bc2) + eps);
+    u.par[p] = w;
+    u.w.publish(p, w);
 }
-
-// BF16 copies of the hidden layers' weights: W [out][in] for the forward products, W^T [in][out] for the backward
-__global__ void k_publish(const float *__restrict__ par, bf16 *w1, bf16 *w2, bf16 *w3, bf16 *w2t, bf16 *w3t)
+// sum over the parts j (in order) of p[j * stride]
+__device__ __forceinline__ float sum_parts(const float *__restrict__ p, int n, int stride)
 {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < HID * HID; i += gridDim.x * blockDim.x) {
-        int o = i / HID, k = i % HID;
-        if (i < HID * NIN) w1[i] = __float2bfloat16_rn(par[OFF_W1 + i]);
-        bf16 a = __float2bfloat16_rn(par[OFF_W2 + i]), b = __float2bfloat16_rn(par[OFF_W3 + i]);
-        w2[i] = a;
-        w3[i] = b;
-        w2t[k * HID + o] = a;
-        w3t[k * HID + o] = b;
+    float acc = 0;
+    for (int j0 = 0; j0 < n; j0 += 16) {
+        float q[16];
+#pragma unroll
+        for (int j = 0; j < 16; j++) q[j] = j0 + j < n ? p[(int64_t)(j0 + j) * stride] : 0.0f;
+#pragma unroll
+        for (int j = 0; j < 16; j++)
+            if (j0 + j < n) acc += q[j];
     }
+    return acc;
 }
+__global__ void __launch_bounds__(256) k_update(Update u)
+{
+    constexpr int HSTRIDE = NOUT * HID + NOUT + 1;
+    if (blockIdx.x < 3 * HID) {
+        __shared__ float red[256];
+        const int l = blockIdx.x / HID, f = blockIdx.x % HID;
+        const bf16 *row = u.dzt[l] + (int64_t)f * u.M;
+        float acc = 0;
+        for (int i0 = threadIdx.x; i0 < u.M; i0 += 8 * 256) {
+            float q[8];
+#pragma unroll
+            for (int j = 0; j < 8; j++) q[j] = i0 + 256 * j < u.M ? __bfloat162float(row[i0 + 256 * j]) : 0.0f;
+#pragma unroll
+            for (int j = 0; j < 8; j++)
+                if (i0 + 256 * j < u.M) acc += q[j];
+        }
+        red[threadIdx.x] = acc;
+        __syncthreads();
+        for (int s = 128; s > 0; s >>= 1) {
+            if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) adam(u, (l == 0 ? OFF_B3 : l == 1 ? OFF_B2 : OFF_B1) + f, red[0]);
+        return;
+    }
+    int q = (blockIdx.x - 3 * HID) * 256 + threadIdx.x;
+    if (q < 2 * HID * HID) {
+        const int l = q / (HID * HID), i = q % (HID * HID);
+        adam(u, (l == 0 ? OFF_W3 : OFF_W2) + i, sum_parts(u.part[l] + i, u.splits, HID * HID));
+        return;
+    }
+    q -= 2 * HID * HID;
+    if (q < HID * NIN) {
+        adam(u, OFF_W1 + q, sum_parts(u.part[2] + q, u.splits, HID * NIN));
+        return;
+    }
+    q -= HID * NIN;
+    if (q < NOUT * HID + NOUT) adam(u, OFF_W4 + q, sum_parts(u.hpart + q, u.nblk, HSTRIDE));
+    else if (q == NOUT * HID + NOUT && u.loss) *u.loss = sum_parts(u.hpart + q, u.nblk, HSTRIDE);
+}
+constexpr int kUpdateBlocks = 3 * HID + (2 * HID * HID + HID * NIN + NOUT * HID + NOUT + 1 + 255) / 256;
 
 // column sums and sums of squares of an [n][w] FP32 array, per block (double, fixed order)
 __global__ void k_moments(const float *__restrict__ x, int64_t n, int w, double *__restrict__ part)
@@ -406,14 +614,6 @@ __global__ void k_moments(const float *__restrict__ x, int64_t n, int w, double 
 }
 
 __global__ void k_read_err(int *err, int *out) { *out = *err; *err = 0; }
-
-template <int N, int EPI>
-void launch_gemm(const Gemm &g, int splits, cudaStream_t s)
-{
-    ensure_dynamic_smem((const void *)k_gemm<N, EPI>, gemm_smem<N>());
-    dim3 grid((g.M + BM - 1) / BM, splits);
-    k_gemm<N, EPI><<<grid, 128, gemm_smem<N>(), s>>>(g);
-}
 
 }  // namespace wsm
 
@@ -482,7 +682,7 @@ void WarmStartNet::set_norm(const float *host)
 
 void WarmStartNet::publish(cudaStream_t s)
 {
-    k_publish<<<64, 256, 0, s>>>(par_.p, w1_.p, w2_.p, w3_.p, w2t_.p, w3t_.p);
+    k_publish<<<(NPAR + 255) / 256, 256, 0, s>>>(par_.p, Weights{w1_.p, w2_.p, w3_.p, w2t_.p, w3t_.p});
 }
 
 void WarmStartNet::add_samples_device(const float *d_x, const float *d_t, int64_t n, cudaStream_t s)
@@ -549,89 +749,59 @@ void WarmStartNet::ensure_batch(int B)
 {
     if (B <= bcap_) return;
     size_t b = (size_t)B;
-    xb_.resize(b * NIN); xbt_.resize(b * NIN);
-    h1_.resize(b * HID); h2_.resize(b * HID); h3_.resize(b * HID); h1t_.resize(b * HID); h2t_.resize(b * HID);
-    dz1_.resize(b * HID); dz2_.resize(b * HID); dz3_.resize(b * HID); dz1t_.resize(b * HID); dz2t_.resize(b * HID);
-    dz3t_.resize(b * HID);
-    tb_.resize(b * NOUT); z1_.resize(b * HID); z2_.resize(b * HID); z3_.resize(b * HID); y_.resize(b * NOUT);
+    xbt_.resize(b * NIN);
+    h1t_.resize(b * HID); h2t_.resize(b * HID);
+    dz1t_.resize(b * HID); dz2t_.resize(b * HID); dz3t_.resize(b * HID);
     int splits = (B + SPLIT_K - 1) / SPLIT_K;
-    part_.resize((size_t)splits * HID * HID);
+    part_.resize((size_t)splits * (2 * HID * HID + HID * NIN));
     hpart_.resize((size_t)((B + 127) / 128) * (NOUT * HID + NOUT + 1));
-    idx_.resize(b);
     bcap_ = B;
 }
 
-// forward over the packed batch xb_ (B rows): z and both layouts of h kept for the backward pass when training
-void WarmStartNet::forward(int B, bool train, cudaStream_t s)
+// One step on a batch of B rows (a multiple of 128; rows idx of the n rows x, t): gradients into grad_, and with lr != 0
+// one Adam step; with loss the sum of the batch's squared errors.
+void WarmStartNet::step(const float *x, const float *t, const int32_t *idx, int64_t n, int B, float lr, float *loss, cudaStream_t s)
 {
     int *err = (int *)loss_.p + 2;
-    Gemm g{};
-    g.M = B; g.kper = 1 << 30; g.err = err; g.ldht = B;
-    g.A = xb_.p; g.lda = NIN; g.B = w1_.p; g.ldb = NIN; g.K = NIN; g.bias = par_.p + OFF_B1;
-    g.zout = train ? z1_.p : nullptr; g.h = h1_.p; g.ht = train ? h1t_.p : nullptr;
-    launch_gemm<HID, EPI_FWD>(g, 1, s);
-    g.A = h1_.p; g.lda = HID; g.B = w2_.p; g.ldb = HID; g.K = HID; g.bias = par_.p + OFF_B2;
-    g.zout = train ? z2_.p : nullptr; g.h = h2_.p; g.ht = train ? h2t_.p : nullptr;
-    launch_gemm<HID, EPI_FWD>(g, 1, s);
-    g.A = h2_.p; g.B = w3_.p; g.bias = par_.p + OFF_B3;
-    g.zout = train ? z3_.p : nullptr; g.h = h3_.p; g.ht = nullptr;
-    launch_gemm<HID, EPI_FWD>(g, 1, s);
-}
-
-// backward over the batch (n valid rows of B) after forward(B, true) and k_head_fwd into y_; fills grad_ and,
-// with apply, takes one Adam step. Returns the batch's mean squared error (reads it back).
-float WarmStartNet::backward_and_step(int B, bool apply, float lr, cudaStream_t s)
-{
-    int *err = (int *)loss_.p + 2;
-    int nblk = (B + 127) / 128;
-    k_head_bwd<<<nblk, 128, 0, s>>>(h3_.p, z3_.p, y_.p, tb_.p, B, B, par_.p, dz3_.p, dz3t_.p, hpart_.p);
-    int hstride = NOUT * HID + NOUT + 1;
-    k_sum_parts<<<4, 128, 0, s>>>(hpart_.p, nblk, NOUT * HID + NOUT, hstride, grad_.p + OFF_W4);  // dW4, db4
-    Gemm g{};
-    g.M = B; g.kper = 1 << 30; g.err = err; g.ldht = B;
-    // dz2 = (dz3 W3) * GELU'(z2), dz1 = (dz2 W2) * GELU'(z1)
-    g.A = dz3_.p; g.lda = HID; g.B = w3t_.p; g.ldb = HID; g.K = HID; g.zin = z2_.p; g.h = dz2_.p; g.ht = dz2t_.p;
-    launch_gemm<HID, EPI_BWD>(g, 1, s);
-    g.A = dz2_.p; g.B = w2t_.p; g.zin = z1_.p; g.h = dz1_.p; g.ht = dz1t_.p;
-    launch_gemm<HID, EPI_BWD>(g, 1, s);
-    // weight gradients: dW_l = dz_l^T h_(l-1), K = the batch split over CTAs
-    int splits = (B + SPLIT_K - 1) / SPLIT_K;
-    Gemm w{};
-    w.M = HID; w.K = B; w.kper = SPLIT_K; w.err = err; w.part = part_.p;
-    w.A = dz3t_.p; w.lda = B; w.B = h2t_.p; w.ldb = B;
-    launch_gemm<HID, EPI_PART>(w, splits, s);
-    k_sum_parts<<<64, 256, 0, s>>>(part_.p, splits, HID * HID, HID * HID, grad_.p + OFF_W3);
-    w.A = dz2t_.p; w.B = h1t_.p;
-    launch_gemm<HID, EPI_PART>(w, splits, s);
-    k_sum_parts<<<64, 256, 0, s>>>(part_.p, splits, HID * HID, HID * HID, grad_.p + OFF_W2);
-    w.A = dz1t_.p; w.B = xbt_.p;
-    launch_gemm<NIN, EPI_PART>(w, splits, s);
-    k_sum_parts<<<8, 256, 0, s>>>(part_.p, splits, HID * NIN, HID * NIN, grad_.p + OFF_W1);
-    k_row_sums<<<HID, 256, 0, s>>>(dz3t_.p, B, grad_.p + OFF_B3);
-    k_row_sums<<<HID, 256, 0, s>>>(dz2t_.p, B, grad_.p + OFF_B2);
-    k_row_sums<<<HID, 256, 0, s>>>(dz1t_.p, B, grad_.p + OFF_B1);
-    if (apply) {
+    const int splits = (B + SPLIT_K - 1) / SPLIT_K, nblk = B / BM;
+    Tile g{};
+    g.x = x; g.t = t; g.idx = idx; g.n = n; g.M = B; g.norm = norm_.p; g.par = par_.p;
+    g.w1 = w1_.p; g.w2 = w2_.p; g.w3 = w3_.p; g.w2t = w2t_.p; g.w3t = w3t_.p;
+    g.xbt = xbt_.p; g.h1t = h1t_.p; g.h2t = h2t_.p; g.dz1t = dz1t_.p; g.dz2t = dz2t_.p; g.dz3t = dz3t_.p;
+    g.hpart = hpart_.p; g.err = err;
+    ensure_dynamic_smem((const void *)k_tile<true>, tile_smem<true>());
+    k_tile<true><<<nblk, kTileThreads, tile_smem<true>(), s>>>(g);
+    float *p3 = part_.p, *p2 = p3 + (size_t)splits * HID * HID, *p1 = p2 + (size_t)splits * HID * HID;
+    Grad w{{dz3t_.p, dz2t_.p, dz1t_.p}, {h2t_.p, h1t_.p, xbt_.p}, {p3, p2, p1}, B, err};
+    ensure_dynamic_smem((const void *)k_wgrad, grad_smem());
+    k_wgrad<<<dim3(splits, 2 * (HID / kGradN) + 1), 256, grad_smem(), s>>>(w);
+    Update u{};
+    u.dzt[0] = dz3t_.p; u.dzt[1] = dz2t_.p; u.dzt[2] = dz1t_.p;
+    u.part[0] = p3; u.part[1] = p2; u.part[2] = p1; u.hpart = hpart_.p;
+    u.M = B; u.splits = splits; u.nblk = nblk;
+    u.grad = grad_.p; u.par = par_.p; u.m = m_.p; u.v = v_.p; u.loss = loss; u.lr = lr;
+    u.w = Weights{w1_.p, w2_.p, w3_.p, w2t_.p, w3t_.p};
+    if (lr != 0.0f) {
         adam_t_++;
-        float bc1 = 1.0f - std::pow(0.9f, (float)adam_t_), bc2 = 1.0f - std::pow(0.999f, (float)adam_t_);
-        k_adam<<<64, 256, 0, s>>>(par_.p, grad_.p, m_.p, v_.p, NPAR, lr, bc1, bc2);
-        publish(s);
+        u.bc1 = 1.0f - std::pow(0.9f, (float)adam_t_);
+        u.bc2 = 1.0f - std::pow(0.999f, (float)adam_t_);
     }
-    return 0.0f;
+    k_update<<<kUpdateBlocks, 256, 0, s>>>(u);
+    cuda_check(cudaGetLastError(), "warm-start training launch");
 }
 
 void WarmStartNet::infer_device(const float *d_x, int64_t n, float *d_y, cudaStream_t s)
 {
     if (n <= 0) return;
-    int64_t done = 0;
-    while (done < n) {
-        int B = (int)std::min<int64_t>(n - done, BMAX);
-        int Bp = (B + 127) / 128 * 128;
-        ensure_batch(Bp);
-        k_pack_inputs<<<(Bp + 127) / 128, 128, 0, s>>>(d_x + done * NIN, nullptr, B, Bp, norm_.p, xb_.p, nullptr, Bp,
-                                                       nullptr, nullptr);
-        forward(Bp, false, s);
-        k_head_fwd<<<(B + 127) / 128, 128, 0, s>>>(h3_.p, B, par_.p, norm_.p, 1, d_y + done * NOUT);
-        done += B;
+    ensure_dynamic_smem((const void *)k_tile<false>, tile_smem<false>());
+    for (int64_t done = 0; done < n;) {  // (one launch up to a thousand million rows)
+        const int M = (int)std::min<int64_t>(n - done, 1 << 30);
+        Tile g{};
+        g.x = d_x + done * NIN; g.n = M; g.M = M; g.norm = norm_.p; g.par = par_.p; g.w1 = w1_.p; g.w2 = w2_.p; g.w3 = w3_.p;
+        g.y = d_y + done * NOUT; g.err = (int *)loss_.p + 2;
+        k_tile<false><<<(M + BM - 1) / BM, kTileThreads, tile_smem<false>(), s>>>(g);
+        cuda_check(cudaGetLastError(), "warm-start inference launch");
+        done += M;
     }
     int e = 0;
     k_read_err<<<1, 1, 0, s>>>((int *)loss_.p + 2, (int *)loss_.p + 3);
@@ -658,10 +828,7 @@ float WarmStartNet::gradients_host(const float *x, const float *t, int64_t n, fl
     DBuf<float> a, b;
     a.upload(x, (size_t)n * NIN, st_);
     b.upload(t, (size_t)n * NOUT, st_);
-    k_pack_inputs<<<(B + 127) / 128, 128, 0, st_>>>(a.p, nullptr, n, B, norm_.p, xb_.p, xbt_.p, B, b.p, tb_.p);
-    forward(B, true, st_);
-    k_head_fwd<<<(B + 127) / 128, 128, 0, st_>>>(h3_.p, B, par_.p, norm_.p, 0, y_.p);
-    backward_and_step(B, false, 0.0f, st_);
+    step(a.p, b.p, nullptr, n, B, 0.0f, nullptr, st_);
     std::vector<float> g(NPAR + 1);
     cuda_check(cudaMemcpyAsync(g.data(), grad_.p, sizeof(float) * NPAR, cudaMemcpyDeviceToHost, st_), "D2H");
     int e = 0;
@@ -689,37 +856,53 @@ float WarmStartNet::train(int steps, int batch, float lr, uint64_t seed)
     cudaEventCreate(&e1);
     cudaEventRecord(e0, st_);
     std::mt19937_64 rng(seed);
-    std::vector<int32_t> perm((size_t)count_);
+    // The next order of the samples is shuffled by a second thread while batches of the current one are launched
+    // (below kShuffleAhead samples shuffling takes less than starting a thread).
+    std::vector<int32_t> perm((size_t)count_), ahead;
     std::iota(perm.begin(), perm.end(), 0);
-    int64_t pos = count_;
-    std::vector<int32_t> idx(B);
+    int64_t pos = count_, shuffles = ((int64_t)steps * B + count_ - 1) / count_;
+    std::future<void> busy;
+    auto next_order = [&]() {
+        if (busy.valid()) {
+            busy.get();
+            perm.swap(ahead);
+        } else {
+            std::shuffle(perm.begin(), perm.end(), rng);
+        }
+        pos = 0;
+        if (--shuffles <= 0 || count_ < kShuffleAhead) return;
+        ahead = perm;
+        try {
+            busy = std::async(std::launch::async, [&] { std::shuffle(ahead.begin(), ahead.end(), rng); });
+        } catch (const std::system_error &) {  // (no thread to be had: shuffled above when its turn comes)
+        }
+    };
+    // The device reads a batch's indices from pinned host memory, out of a ring of slots, so that the host runs ahead.
     HostPinned<int32_t> hidx;
-    hidx.resize((size_t)B * 2);
-    int nblk = (B + 127) / 128, hstride = NOUT * HID + NOUT + 1;
+    hidx.resize((size_t)B * kIdxSlots);
+    struct Drain {  // (an error leaves no kernel behind that reads a slot)
+        cudaStream_t s;
+        ~Drain() { cudaStreamSynchronize(s); }
+    } drain{st_};
+    cudaEvent_t free_ev[kIdxSlots];
+    for (auto &e : free_ev) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
     DBuf<float> losses;
     int tail = std::max(1, steps / 10);
     losses.resize((size_t)tail);
     losses.zero(st_);
     for (int it = 0; it < steps; it++) {
-        for (int r = 0; r < B; r++) {
-            if (pos >= count_) {
-                std::shuffle(perm.begin(), perm.end(), rng);
-                pos = 0;
-            }
-            idx[r] = perm[pos++];
+        const int slot = it % kIdxSlots;
+        int32_t *hb = hidx.p + (size_t)slot * B;
+        if (it >= kIdxSlots) cuda_check(cudaEventSynchronize(free_ev[slot]), "cudaEventSynchronize");
+        for (int r = 0; r < B;) {
+            if (pos >= count_) next_order();
+            const int take = (int)std::min<int64_t>(B - r, count_ - pos);
+            std::memcpy(hb + r, perm.data() + pos, sizeof(int32_t) * take);
+            r += take;
+            pos += take;
         }
-        int32_t *hb = hidx.p + (it & 1) * B;
-        cuda_check(cudaStreamSynchronize(st_), "cudaStreamSynchronize");  // the pinned slot is free again
-        std::memcpy(hb, idx.data(), sizeof(int32_t) * B);
-        cuda_check(cudaMemcpyAsync(idx_.p, hb, sizeof(int32_t) * B, cudaMemcpyHostToDevice, st_), "H2D");
-        k_pack_inputs<<<nblk, 128, 0, st_>>>(dx_.p, idx_.p, count_, B, norm_.p, xb_.p, xbt_.p, B, dt_.p, tb_.p);
-        forward(B, true, st_);
-        k_head_fwd<<<nblk, 128, 0, st_>>>(h3_.p, B, par_.p, norm_.p, 0, y_.p);
-        backward_and_step(B, true, lr, st_);
-        if (it >= steps - tail) {
-            // the batch loss: the last slot of the head partials, summed into the ring of final losses
-            k_sum_parts<<<1, 1, 0, st_>>>(hpart_.p + hstride - 1, nblk, 1, hstride, losses.p + (it - (steps - tail)));
-        }
+        step(dx_.p, dt_.p, hb, count_, B, lr, it >= steps - tail ? losses.p + (it - (steps - tail)) : nullptr, st_);
+        cuda_check(cudaEventRecord(free_ev[slot], st_), "cudaEventRecord");
     }
     std::vector<float> hl((size_t)tail);
     losses.download(hl.data(), (size_t)tail, st_);
@@ -733,6 +916,7 @@ float WarmStartNet::train(int steps, int batch, float lr, uint64_t seed)
     train_ms += ms;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
+    for (auto &q : free_ev) cudaEventDestroy(q);
     if (e) throw Failure(IFEA_CUDA_ERROR, "Warm-start network: a tensor-core wait timed out.");
     double l = 0;
     for (float v : hl) l += v;

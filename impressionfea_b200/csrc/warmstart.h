@@ -52,8 +52,7 @@ class WarmStartNet {
 
   private:
     void publish(cudaStream_t s);
-    void forward(int B, bool train, cudaStream_t s);
-    float backward_and_step(int B, bool apply, float lr, cudaStream_t s);
+    void step(const float *x, const float *t, const int32_t *idx, int64_t n, int B, float lr, float *loss, cudaStream_t s);
     void ensure_batch(int B);
 
     cudaStream_t st_ = nullptr;
@@ -62,9 +61,10 @@ class WarmStartNet {
     DBuf<__nv_bfloat16> w1_, w2_, w3_, w2t_, w3t_;
     // batch workspace
     int bcap_ = 0;
-    DBuf<__nv_bfloat16> xb_, xbt_, h1_, h2_, h3_, h1t_, h2t_, dz1_, dz2_, dz3_, dz1t_, dz2t_, dz3t_;
-    DBuf<float> tb_, z1_, z2_, z3_, y_, part_, hpart_, loss_;
-    DBuf<int32_t> idx_;
+    static constexpr int kIdxSlots = 8;        // batches the host runs ahead of the device
+    static constexpr int kShuffleAhead = 4096;  // samples from which the next order is made on another thread
+    DBuf<__nv_bfloat16> xbt_, h1t_, h2t_, dz1t_, dz2t_, dz3t_;  // [feature][row]
+    DBuf<float> part_, hpart_, loss_;
     // training set
     DBuf<float> dx_, dt_;
     int64_t count_ = 0, cap_ = 0;
