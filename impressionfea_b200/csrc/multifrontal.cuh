@@ -31,6 +31,8 @@ namespace mf {
 constexpr int PW = 64;  // panel width
 constexpr int UT = 64;  // update tile
 constexpr int SST = UT + 4;  // row stride of the k-major operand tiles in shared memory (16-byte aligned rows)
+constexpr int KC = 32;       // k rows of a tile that is read while the next ones are on their way
+constexpr int KST = KC + 4;  // row stride of an operand tile held by columns, KC entries each
 
 template <typename T>
 struct Dev {
@@ -47,57 +49,78 @@ struct Dev {
 constexpr int kWideM = 192;
 constexpr int kWideMinCols = 0;
 
-// Rows (or columns) of a 64-wide tile owned by thread index t (0..15): four consecutive ones in single precision
-// (one 16-byte shared-memory load), pairs {2t, 2t + 1} and {2t + 32, 2t + 33} in double precision (two 16-byte
-// loads that keep a half-warp on consecutive banks).
-__device__ __forceinline__ int tile_row(float, int t, int a) { return 4 * t + a; }
-__device__ __forceinline__ int tile_row(double, int t, int a) { return 2 * t + (a & 1) + 32 * (a >> 1); }
-__device__ __forceinline__ void lds4(const float *row, int t, float (&v)[4])
+// acc += A^T B over kn steps of two k-major 64-wide tiles by 256 threads (a CTA, or a third of one), sixteen entries a thread: acc[a][b] is
+// entry (acc_row(T(), a), acc_col(T(), b)).
+//
+// In double precision on the tensor cores (mma.sync m8n8k4, the FP64 form this chip has: 36.9 TFLOP/s measured, 31.2
+// with FMA instructions): a warp owns 32 x 16, and a step of four k reads six doubles a lane from shared memory for
+// eight MMAs. A thread's 4 x 4 block of FMAs reads 32 for the same work, which kept the shared-memory pipe as busy as
+// the arithmetic. Rows 68 doubles apart put a half-warp's 4 rows x 4 columns on distinct banks, for an operand tile
+// held either way round. kn is rounded up to a multiple of four: the rows of both tiles up to there have to be zero.
+// In single precision a thread owns four consecutive rows and columns (one 16-byte load each a step).
+__device__ __forceinline__ int acc_row(float, int a) { return 4 * (threadIdx.x % 16) + a; }
+__device__ __forceinline__ int acc_col(float, int b) { return 4 * (threadIdx.x / 16 % 16) + b; }
+__device__ __forceinline__ int acc_row(double, int a) { return 32 * ((threadIdx.x >> 5) & 1) + 8 * a + ((threadIdx.x & 31) >> 2); }
+__device__ __forceinline__ int acc_col(double, int b)
 {
-    float4 q = *reinterpret_cast<const float4 *>(row + 4 * t);
-    v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
-}
-__device__ __forceinline__ void lds4(const double *row, int t, double (&v)[4])
-{
-    double2 q0 = *reinterpret_cast<const double2 *>(row + 2 * t), q1 = *reinterpret_cast<const double2 *>(row + 2 * t + 32);
-    v[0] = q0.x, v[1] = q0.y, v[2] = q1.x, v[3] = q1.y;
+    return 16 * ((threadIdx.x >> 6) & 3) + 8 * (b >> 1) + 2 * (threadIdx.x & 3) + (b & 1);
 }
 
-// acc += A^T B over kn steps of two k-major 64-wide tiles: thread (tx, ty) owns rows tile_row(tx, 0..3) of A's
-// columns and tile_row(ty, 0..3) of B's, so each step is two or four vector loads for sixteen FMAs.
-// Asynchronous copy of a 64 x 64 k-major tile into shared memory for a 256-thread CTA (cp.async, no register
-// staging, so all sixteen copies of a thread are in flight together): element (k, r) is src[k * ld + r] when
-// k < kn and r < rn, zero otherwise. tile_wait() completes every copy the thread issued.
-template <typename T>
-__device__ __forceinline__ void tile_fetch(T (*dst)[SST], const T *__restrict__ src, int64_t ld, int kn, int rn)
+__device__ __forceinline__ void tile_mma(const float *A, const float *B, int kn, float (&acc)[4][4])
 {
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        int q = threadIdx.x + 256 * i, r = q & 63, k = q >> 6;
-        bool ok = k < kn && r < rn;
-        const T *g = ok ? src + (int64_t)k * ld + r : src;
-        unsigned sa = (unsigned)__cvta_generic_to_shared(&dst[k][r]);
-        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(sa), "l"(g), "n"((int)sizeof(T)),
-                     "r"(ok ? (int)sizeof(T) : 0));
-    }
-    asm volatile("cp.async.commit_group;\n" ::);
-}
-__device__ __forceinline__ void tile_wait() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
-
-template <typename T>
-__device__ __forceinline__ void tile_mma(const T (*A)[SST], const T (*B)[SST], int kn, int tx, int ty, T (&acc)[4][4])
-{
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16 % 16;
 #pragma unroll 4
     for (int k = 0; k < kn; k++) {
-        T a[4], b[4];
-        lds4(A[k], tx, a);
-        lds4(B[k], ty, b);
+        const float4 p = *reinterpret_cast<const float4 *>(A + k * SST + 4 * tx), q = *reinterpret_cast<const float4 *>(B + k * SST + 4 * ty);
+        const float a[4] = {p.x, p.y, p.z, p.w}, b[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
             for (int j = 0; j < 4; j++) acc[i][j] = fma(a[i], b[j], acc[i][j]);
     }
 }
+// BT: B is held by columns, B[column * KST + k]
+template <bool BT = false>
+__device__ __forceinline__ void tile_mma(const double *A, const double *B, int kn, double (&acc)[4][4])
+{
+    const int lane = threadIdx.x & 31, kq = lane & 3, r = 32 * ((threadIdx.x >> 5) & 1) + (lane >> 2),
+              c = 16 * ((threadIdx.x >> 6) & 3) + (lane >> 2);
+#pragma unroll 4
+    for (int k = 0; k < kn; k += 4) {
+        double a[4], b[2];
+#pragma unroll
+        for (int i = 0; i < 4; i++) a[i] = A[(k + kq) * SST + r + 8 * i];
+#pragma unroll
+        for (int j = 0; j < 2; j++) b[j] = BT ? B[(c + 8 * j) * KST + k + kq] : B[(k + kq) * SST + c + 8 * j];
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+                asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                    : "+d"(acc[i][2 * j]), "+d"(acc[i][2 * j + 1])
+                    : "d"(a[i]), "d"(b[j]));
+    }
+}
+
+// Asynchronous copy of a KR x 64 k-major tile into shared memory by 256 threads (cp.async, no register
+// staging, so all copies of a thread are in flight together): element (k, r) is src[k * ld + r] when
+// k < kn and r < rn, zero otherwise. tile_wait<N>() completes all but the N last copies the thread issued.
+template <typename T, int KR = PW>
+__device__ __forceinline__ void tile_copy(T *dst, const T *__restrict__ src, int64_t ld, int kn, int rn)
+{
+#pragma unroll
+    for (int i = 0; i < KR / 4; i++) {
+        int q = threadIdx.x % 256 + 256 * i, r = q & 63, k = q >> 6;
+        bool ok = k < kn && r < rn;
+        const T *g = ok ? src + (int64_t)k * ld + r : src;
+        unsigned sa = (unsigned)__cvta_generic_to_shared(dst + k * SST + r);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(sa), "l"(g), "n"((int)sizeof(T)),
+                     "r"(ok ? (int)sizeof(T) : 0));
+    }
+}
+__device__ __forceinline__ void tile_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N = 0>
+__device__ __forceinline__ void tile_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 template <typename T>
 static __global__ void k_scatter(int64_t n, const int64_t *__restrict__ dst, const int32_t *__restrict__ src,
@@ -402,8 +425,8 @@ static __global__ void __launch_bounds__(256) k_panel_trsm(Dev<T> D, const int32
 {
     extern __shared__ __align__(16) unsigned char shm_raw[];
     T *shm = (T *)shm_raw;
-    T (*Ft)[SST] = (T (*)[SST])shm;             // Ft[l][row]
-    T (*Di)[SST] = (T (*)[SST])(shm + PW * SST);  // Di[l][k] = Dinv[k][l]
+    T *Ft = shm;             // Ft(l, row)
+    T *Di = shm + PW * SST;  // Di(l, k) = Dinv(k, l)
     int s = fronts[blockIdx.y];
     int ms = D.m[s], w = min(PW, D.ncol[s] - k0);
     int rbeg = k0 + w + blockIdx.x * PW;
@@ -411,18 +434,18 @@ static __global__ void __launch_bounds__(256) k_panel_trsm(Dev<T> D, const int32
     int rows = min(PW, ms - rbeg);
     T *F = D.F + D.front_off[s];
     const T *Inv = D.Inv + D.inv_off[s] + (int64_t)(k0 / PW) * PW * PW;
-    tile_fetch(Di, Inv, PW, w, PW);  // column l of the column-major inverse
-    tile_fetch(Ft, F + (int64_t)k0 * ms + rbeg, ms, w, rows);
+    tile_copy(Di, Inv, PW, w, PW);  // column l of the column-major inverse
+    tile_copy(Ft, F + (int64_t)k0 * ms + rbeg, ms, w, rows);
+    tile_commit();
     tile_wait();
     __syncthreads();
-    int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
     T acc[4][4];
     for (int a = 0; a < 4; a++)
         for (int b = 0; b < 4; b++) acc[a][b] = T(0);
-    tile_mma<T>(Ft, Di, w, tx, ty, acc);
+    tile_mma(Ft, Di, w, acc);
     for (int b = 0; b < 4; b++)
         for (int a = 0; a < 4; a++) {
-            int rr = tile_row(T(), tx, a), k = tile_row(T(), ty, b);
+            int rr = acc_row(T(), a), k = acc_col(T(), b);
             if (rr < rows && k < w) F[(int64_t)(k0 + k) * ms + rbeg + rr] = acc[a][b];
         }
 }
@@ -434,6 +457,7 @@ static __global__ void __launch_bounds__(256) k_panel_trsm(Dev<T> D, const int32
 // in X's unused upper triangle), then X21 = -X22 T (k_xinv_gemm<1>). The tasks of one pass are listed on the host;
 // one CTA per task, each thread a 4 x 4 register block. The passes run on a side stream, overlapping the
 // factorisation of the levels above (only the solves read X).
+constexpr int kPairBuf = KC * SST + PW * KST;  // an operand pair of KC k rows, the second held either way
 struct XTask {
     int s, bi, bj, kb0, kb1, slot, nslot, pad;  // front, output block, block range, partial slots
 };
@@ -451,6 +475,8 @@ static __global__ void k_xinv_diag(Dev<T> D, const XTask *__restrict__ tasks)
     }
 }
 
+// (B200, 57k equations in FP64, all passes: 9.4 ms with FMA tiles loaded between two barriers, 5.7 ms on the tensor
+// cores with the next half block on its way.)
 // k_xinv_gemm computes one 64 x 64 output tile over the block range [kb0, kb1): in place when slot < 0, else as a
 // partial tile into the workspace, summed by k_xinv_reduce in slot order (long ranges are split so that no CTA
 // runs much longer than the others).
@@ -465,44 +491,59 @@ __device__ __forceinline__ void xinv_store(T *X, int nc, int r0, int c0, int r, 
 }
 
 template <typename T, int PASS>
-static __global__ void __launch_bounds__(256) k_xinv_gemm(Dev<T> D, const XTask *__restrict__ tasks, T *__restrict__ W)
+static __global__ void __launch_bounds__(256, 3) k_xinv_gemm(Dev<T> D, const XTask *__restrict__ tasks, T *__restrict__ W)
 {
     extern __shared__ __align__(16) unsigned char shm_raw[];
     T *shm = (T *)shm_raw;
-    T (*A)[SST] = (T (*)[SST])shm;             // A[k][r]
-    T (*B)[SST] = (T (*)[SST])(shm + PW * SST);  // B[k][c]
     XTask tk = tasks[blockIdx.x];
     int s = tk.s, bi = tk.bi, bj = tk.bj;
     int ms = D.m[s], nc = D.ncol[s];
     const T *F = D.F + D.front_off[s];
     T *X = D.Xinv + D.xinv_off[s];
     int r0 = bi * PW, c0 = bj * PW, wr = min(PW, nc - r0), wc = min(PW, nc - c0);
-    int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
     T acc[4][4];
     for (int a = 0; a < 4; a++)
         for (int b = 0; b < 4; b++) acc[a][b] = T(0);
-    for (int bk = tk.kb0; bk < tk.kb1; bk++) {
-        int k0 = bk * PW, wk = min(PW, nc - k0);
-        __syncthreads();
-        for (int t = threadIdx.x; t < PW * PW; t += blockDim.x) {
-            int lo = t % PW, hi = t / PW;  // lo runs along contiguous memory
-            // A(r = lo, k = hi): pass 0 L(bi, bk) from the front, pass 1 X(bi, bk)
-            bool oka = lo < wr && hi < wk;
-            A[hi][lo] = !oka       ? T(0)
-                        : PASS == 0 ? F[(int64_t)(k0 + hi) * ms + r0 + lo]
-                                    : X[(int64_t)(k0 + hi) * nc + r0 + lo];
-            if (PASS == 0)  // B(k = lo, c = hi) = X(bk, bj)
-                B[lo][hi] = (lo < wk && hi < wc) ? X[(int64_t)(c0 + hi) * nc + k0 + lo] : T(0);
-            else  // B(k = hi, c = lo) = T(bk, bj), stored at X(c0 + c, k0 + k)
-                B[hi][lo] = (hi < wk && lo < wc) ? X[(int64_t)(k0 + hi) * nc + c0 + lo] : T(0);
+    // Half a block (32 k) at a time through two buffers, the copies of one half under the products of the other
+    constexpr bool BT = PASS == 0 && std::is_same<T, double>::value;  // B as it lies in memory, [column][k]
+    const int half0 = 2 * tk.kb0, half1 = (min(nc, tk.kb1 * PW) + KC - 1) / KC;
+    auto fetch = [&](int h) {
+        T *A = shm + (h & 1) * kPairBuf, *B = A + KC * SST;
+        const int k0 = h * KC, wk = min(KC, nc - k0);
+        // A(k, r): pass 0 L(bi, bk) from the front, pass 1 X(bi, bk)
+        if (PASS == 0) tile_copy<T, KC>(A, F + (int64_t)k0 * ms + r0, ms, wk, wr);
+        else tile_copy<T, KC>(A, X + (int64_t)k0 * nc + r0, nc, wk, wr);
+        // B(k, c): pass 0 X(bk, bj), contiguous along k; pass 1 T(bk, bj), stored at X(c0 + c, k0 + k)
+        if (PASS == 1) {
+            tile_copy<T, KC>(B, X + (int64_t)k0 * nc + c0, nc, wk, wc);
+        } else {
+#pragma unroll
+            for (int i = 0; i < KC / 4; i++) {
+                const int q = threadIdx.x + 256 * i, k = q % KC, c = q / KC;
+                const bool ok = k < wk && c < wc;
+                const T *g = ok ? X + (int64_t)(c0 + c) * nc + k0 + k : X;
+                const unsigned sa = (unsigned)__cvta_generic_to_shared(B + (BT ? c * KST + k : k * SST + c));
+                asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(sa), "l"(g), "n"((int)sizeof(T)),
+                             "r"(ok ? (int)sizeof(T) : 0));
+            }
         }
+        tile_commit();
+    };
+    fetch(half0);
+    for (int h = half0; h < half1; h++) {
+        const T *A = shm + (h & 1) * kPairBuf, *B = A + KC * SST;
+        if (h + 1 < half1) fetch(h + 1);
+        else tile_commit();
+        tile_wait<1>();
         __syncthreads();
-        tile_mma<T>(A, B, PW, tx, ty, acc);
+        if constexpr (BT) tile_mma<true>(A, B, KC, acc);
+        else tile_mma(A, B, KC, acc);
+        __syncthreads();
     }
     T *Wt = tk.slot >= 0 ? W + (int64_t)tk.slot * PW * PW : nullptr;
     for (int b = 0; b < 4; b++)
         for (int a = 0; a < 4; a++) {
-            int r = tile_row(T(), tx, a), c = tile_row(T(), ty, b);
+            int r = acc_row(T(), a), c = acc_col(T(), b);
             if (Wt)
                 Wt[c * PW + r] = acc[a][b];
             else if (r < wr && c < wc)
@@ -587,75 +628,177 @@ static __global__ void __launch_bounds__(256) k_mirror(Dev<T> D, const int32_t *
     }
 }
 
-// Trailing update of every listed front by its pivot columns [k0, k0 + kd), kd = min(kdepth, ncol - k0):
-// F22 -= L21 L21^T on the 64 x 64 lower tiles of the region of rows and columns from rs = k0 + kd on (k-major
-// operand tiles in shared memory, each thread a 4 x 4 register block, the kd columns taken 64 at a time).
-// part 0: the whole region; part 1: its first 64 columns (the next panel's, which the next panel step needs
-// first); part 2: its columns from rs + 64 on (applied on a second stream while the next panel is factorised).
-// Parts 1 and 2 stop at column min(ncol, col_end): the pivot columns of the current super-panel.
+template <int GROUPS>
+__device__ __forceinline__ void group_sync()
+{
+    if (GROUPS == 1) __syncthreads();
+    else asm volatile("bar.sync %0, 256;" ::"r"(1 + (int)threadIdx.x / 256) : "memory");
+}
+
+// Trailing updates F22 -= L21 L21^T, on 64 x 64 lower tiles: the tile of front F at rows ri.. and columns cj.. by the kd
+// pivot columns from k0; columns from ce on stay.
 template <typename T>
-static __global__ void __launch_bounds__(256) k_update(Dev<T> D, const int32_t *__restrict__ fronts, int k0, int kdepth,
-                                                       int col_end, int part)
+struct UTile {
+    T *F;
+    int ms, k0, kd, ri, cj, ce;
+};
+template <typename T>
+__device__ __forceinline__ void update_fetch(const UTile<T> &u, int c, T *buf)
+{
+    const T *col = u.F + (int64_t)(u.k0 + c * KC) * u.ms;
+    tile_copy<T, KC>(buf, col + u.ri, u.ms, u.kd - c * KC, u.ms - u.ri);
+    tile_copy<T, KC>(buf + KC * SST, col + u.cj, u.ms, u.kd - c * KC, u.ms - u.cj);
+}
+// 32 pivot columns at a time through two buffers, the copies of one half under the products of the other. The tile's
+// first half is on its way into buffer `cur` already; under the last products `next` sends the following tile's first
+// half to the other buffer. Returns that buffer. GROUPS: the CTA's groups of 256 threads have tiles of their own.
+template <typename T, int GROUPS, typename Next>
+__device__ __forceinline__ int update_tile(const UTile<T> &u, T *sh, int cur, Next next)
+{
+    T acc[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) acc[a][b] = T(0);
+    for (int k = 0, c = 0; k < u.kd; k += KC, c++) {
+        T *buf = sh + cur * 2 * KC * SST;
+        cur ^= 1;
+        if (k + KC < u.kd) update_fetch(u, c + 1, sh + cur * 2 * KC * SST);
+        else next(sh + cur * 2 * KC * SST);
+        tile_commit();
+        tile_wait<1>();
+        group_sync<GROUPS>();
+        tile_mma(buf, buf + KC * SST, min(KC, u.kd - k), acc);
+        group_sync<GROUPS>();
+    }
+    // old values, eight in flight at a time (the others that share the SM multiply meanwhile)
+    const bool inside = u.ri > u.cj && u.ri + UT <= u.ms && u.cj + UT <= u.ce;
+#pragma unroll
+    for (int h = 0; h < 4; h += 2) {
+        T old[2][4];
+        T *out = u.F + (int64_t)(u.cj + acc_col(T(), h)) * u.ms + u.ri + acc_row(T(), 0);
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                const int gi = u.ri + acc_row(T(), a), gj = u.cj + acc_col(T(), h + b);
+                if (inside || (gi < u.ms && gj < u.ce && gi >= gj)) old[b][a] = out[b * u.ms + acc_row(T(), a) - acc_row(T(), 0)];
+            }
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                const int gi = u.ri + acc_row(T(), a), gj = u.cj + acc_col(T(), h + b);
+                if (inside || (gi < u.ms && gj < u.ce && gi >= gj)) out[b * u.ms + acc_row(T(), a) - acc_row(T(), 0)] = old[b][a] - acc[a][h + b];
+            }
+    }
+    return cur;
+}
+template <typename T>
+__device__ __forceinline__ void update_one(const UTile<T> &u, T *sh)
+{
+    update_fetch(u, 0, sh);
+    tile_commit();
+    update_tile<T, 1>(u, sh, 0, [](T *) {});
+}
+__device__ __forceinline__ void lower_tile(int t, int &ti, int &tj)  // tile t of a lower triangle, row by row
+{
+    ti = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while ((ti + 1) * (ti + 2) / 2 <= t) ti++;
+    while (ti * (ti + 1) / 2 > t) ti--;
+    tj = t - ti * (ti + 1) / 2;
+}
+
+// Inside a super-panel, after a panel of kdepth columns: its region up to column min(ncol, col_end).
+// part 1: the first 64 columns (the next panel's, which the next panel step needs first); part 2: the columns from
+// rs + 64 on (applied on a second stream while the next panel is factorised).
+template <typename T>
+static __global__ void __launch_bounds__(256, 3) k_update(Dev<T> D, const int32_t *__restrict__ fronts, int k0, int kdepth,
+                                                          int col_end, int part)
 {
     extern __shared__ __align__(16) unsigned char sh_raw[];
-    T *sh = (T *)sh_raw;
-    T (*Ai)[SST] = (T (*)[SST])sh;
-    T (*Aj)[SST] = (T (*)[SST])(sh + PW * SST);
-    int s = fronts[blockIdx.y];
-    int ms = D.m[s], kd = min(kdepth, D.ncol[s] - k0);
+    const int s = fronts[blockIdx.y], ms = D.m[s], kd = min(kdepth, D.ncol[s] - k0);
     if (kd <= 0) return;
-    int rs = k0 + kd, nt = ms - rs;
-    int ce = part == 0 ? ms : min(ms, min(col_end, D.ncol[s]));
+    const int rs = k0 + kd, nt = ms - rs, ce = min(ms, min(col_end, D.ncol[s]));
     if (nt <= 0 || ce <= rs) return;
-    T *F = D.F + D.front_off[s];
-    int nti = (nt + UT - 1) / UT, nct = (ce - rs + UT - 1) / UT;
-    int ntiles = part == 0 ? nti * (nti + 1) / 2 : part == 1 ? nti : (nct - 1) * nti - (nct - 1) * nct / 2;
-    int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    const int nti = (nt + UT - 1) / UT, nct = (ce - rs + UT - 1) / UT;
+    const int ntiles = part == 1 ? nti : (nct - 1) * nti - (nct - 1) * nct / 2;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        int ti, tj;
-        if (part == 1) {
-            ti = t, tj = 0;
-        } else if (part == 2) {  // column tiles 1 .. nct - 1, rows from the diagonal down
+        int ti = t, tj = 0;
+        if (part == 2) {  // column tiles 1 .. nct - 1, rows from the diagonal down
             int rem = t;
             tj = 1;
             while (rem >= nti - tj) rem -= nti - tj++;
             ti = tj + rem;
-        } else {
-            ti = (int)((sqrt(8.0 * t + 1.0) - 1.0) * 0.5);
-            while ((ti + 1) * (ti + 2) / 2 <= t) ti++;
-            while (ti * (ti + 1) / 2 > t) ti--;
-            tj = t - ti * (ti + 1) / 2;
         }
-        int ri0 = rs + ti * UT, cj0 = rs + tj * UT;
-        T old[4][4], acc[4][4];
-#pragma unroll
-        for (int a = 0; a < 4; a++)
-#pragma unroll
-            for (int b = 0; b < 4; b++) acc[a][b] = T(0);
-        for (int kc = 0; kc < kd; kc += PW) {
-            int kn = min(PW, kd - kc);
-            // operand copies (and, on the first chunk, the output loads) all in flight at once
-            __syncthreads();
-            tile_fetch(Ai, F + (int64_t)(k0 + kc) * ms + ri0, ms, kn, ms - ri0);
-            tile_fetch(Aj, F + (int64_t)(k0 + kc) * ms + cj0, ms, kn, ms - cj0);
-            if (kc == 0) {
-#pragma unroll
-                for (int b = 0; b < 4; b++)
-#pragma unroll
-                    for (int a = 0; a < 4; a++) {
-                        int gi = ri0 + tile_row(T(), tx, a), gj = cj0 + tile_row(T(), ty, b);
-                        old[a][b] = (gi < ms && gj < ce && gi >= gj) ? F[(int64_t)gj * ms + gi] : T(0);
-                    }
-            }
-            tile_wait();
-            __syncthreads();
-            tile_mma<T>(Ai, Aj, kn, tx, ty, acc);
-        }
-        for (int b = 0; b < 4; b++)
-            for (int a = 0; a < 4; a++) {
-                int gi = ri0 + tile_row(T(), tx, a), gj = cj0 + tile_row(T(), ty, b);
-                if (gi < ms && gj < ce && gi >= gj) F[(int64_t)gj * ms + gi] = old[a][b] - acc[a][b];
-            }
+        update_one(UTile<T>{D.F + D.front_off[s], ms, k0, kd, rs + ti * UT, rs + tj * UT, ce}, (T *)sh_raw);
+    }
+}
+
+// The end of a super-panel: every listed front's whole region by its up to `depth` pivot columns from k0, the fronts'
+// tiles as one sequence (front f owns tstart[f] ..), so that no CTA is bound to a small front while others work on a
+// large one. k_update_next: the tiles of the next super-panel's columns, which its panels wait for, a tile a CTA.
+// k_update_rest: all others, beside the next super-panel's chain of panels. A panel's CTA needs an SM's registers to
+// itself and would wait for the whole update if each SM held a part of it: so its CTAs fill an SM each (three groups of
+// 256 threads with a tile each) and the host launches them on fewer SMs than there are.
+// The 57k-equation FP64 factor (B200): one launch over the whole region, 65 CTAs a front whatever its size, four CTAs an
+// SM where three fit and the next panels after it, factorised in 38 ms; tiles in one sequence 32 ms; beside the chain
+// 27.7 ms. Three tiles at work on an SM reach 18 TFLOP/s on 128 SMs (57% of the pipe's rate while an SM works).
+// next_tiles: column tiles of a front's next super-panel, none once its pivot columns are done.
+constexpr int kRestGroups = 3, kRestThreads = 256 * kRestGroups;
+__host__ __device__ inline int next_tiles(int ncol, int rs, int depth)
+{
+    return ncol > rs ? ((ncol < rs + depth ? ncol : rs + depth) - rs + UT - 1) / UT : 0;
+}
+template <bool NEXT, typename T>
+__device__ __forceinline__ UTile<T> update_seq(const Dev<T> &D, const int32_t *__restrict__ fronts,
+                                               const int32_t *__restrict__ tstart, int nf, int k0, int depth, int g)
+{
+    int lo = 0, hi = nf - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (tstart[mid] <= g) lo = mid;
+        else hi = mid - 1;
+    }
+    const int s = fronts[lo], ms = D.m[s], nc = D.ncol[s], kd = min(depth, nc - k0), rs = k0 + kd;
+    const int nti = (ms - rs + UT - 1) / UT, na = next_tiles(nc, rs, depth);
+    int t = g - tstart[lo], ti, tj;
+    if (NEXT) {  // column tiles 0 .. na - 1, rows from the diagonal down
+        tj = 0;
+        while (t >= nti - tj) t -= nti - tj++;
+        ti = tj + t;
+    } else {
+        lower_tile(t, ti, tj);
+        ti += na, tj += na;
+    }
+    return UTile<T>{D.F + D.front_off[s], ms, k0, kd, rs + ti * UT, rs + tj * UT, ms};
+}
+template <typename T>
+static __global__ void __launch_bounds__(256, 3) k_update_next(Dev<T> D, const int32_t *__restrict__ fronts,
+                                                               const int32_t *__restrict__ tstart, int nf, int k0, int depth)
+{
+    extern __shared__ __align__(16) unsigned char sh_raw[];
+    update_one(update_seq<true>(D, fronts, tstart, nf, k0, depth, blockIdx.x), (T *)sh_raw);
+}
+template <typename T>
+static __global__ void __launch_bounds__(kRestThreads, 1) k_update_rest(Dev<T> D, const int32_t *__restrict__ fronts,
+                                                                        const int32_t *__restrict__ tstart, int nf, int k0, int depth)
+{
+    extern __shared__ __align__(16) unsigned char sh_raw[];
+    const int grp = threadIdx.x / 256, total = tstart[nf], step = gridDim.x * kRestGroups;
+    T *sh = (T *)sh_raw + grp * 4 * KC * SST;
+    int g = blockIdx.x + gridDim.x * grp, cur = 0;
+    if (g >= total) return;
+    UTile<T> u = update_seq<false>(D, fronts, tstart, nf, k0, depth, g), v = u;
+    update_fetch(u, 0, sh);
+    tile_commit();
+    for (; g < total; g += step) {
+        const bool more = g + step < total;
+        if (more) v = update_seq<false>(D, fronts, tstart, nf, k0, depth, g + step);
+        cur = update_tile<T, kRestGroups>(u, sh, cur, [&](T *buf) {
+            if (more) update_fetch(v, 0, buf);
+        });
+        u = v;
     }
 }
 
@@ -1045,7 +1188,8 @@ public:
     struct SpStep {  // one super-panel's trailing update within a level
         int tc_off = 0, tc_cnt = 0, tc_grid = 0, tc_rb = 0;  // tensor-core fronts: list, CTAs, most row blocks
         int tc_toff = 0;                                     // their tile-sequence prefix (tc_cnt + 1 entries)
-        int si_off = 0, si_cnt = 0, si_tiles = 0;            // the other fronts: list, most 64 x 64 tiles of one
+        int si_off = 0, si_cnt = 0;                          // the other fronts: list, then the prefixes of their tiles
+        int si_next = 0, si_rest = 0;                        // (si_cnt + 1 entries each): next super-panel's, all others
     };
     explicit MfSolverT(cudaStream_t s) : st_(s)
     {
@@ -1057,6 +1201,8 @@ public:
         cuda_check(cudaStreamCreateWithFlags(&cap_, cudaStreamNonBlocking), "cudaStreamCreate");
         cuda_check(cudaStreamCreateWithFlags(&side_, cudaStreamNonBlocking), "cudaStreamCreate");
         cuda_check(cudaStreamCreateWithFlags(&ahead_, cudaStreamNonBlocking), "cudaStreamCreate");
+        cuda_check(cudaStreamCreateWithFlags(&bulk_, cudaStreamNonBlocking), "cudaStreamCreate");
+        for (cudaEvent_t *e : {&chain_ev_, &bulk_ev_}) cuda_check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "cudaEventCreate");
         int lo = 0;
         cuda_check(cudaDeviceGetStreamPriorityRange(&lo, &prio_hi_), "cudaDeviceGetStreamPriorityRange");
         cuda_check(cudaEventCreateWithFlags(&trsm_ev_, cudaEventDisableTiming), "cudaEventCreate");
@@ -1076,6 +1222,9 @@ public:
         for (auto &e : rest_ev_)
             if (e) cudaEventDestroy(e);
         if (ahead_) cudaStreamDestroy(ahead_);
+        if (bulk_) cudaStreamDestroy(bulk_);
+        if (chain_ev_) cudaEventDestroy(chain_ev_);
+        if (bulk_ev_) cudaEventDestroy(bulk_ev_);
         if (cap_) cudaStreamDestroy(cap_);
         if (descr_) cusparseDestroyMatDescr(descr_);
         if (hsp_) cusolverSpDestroy(hsp_);
@@ -1303,6 +1452,8 @@ public:
         dev_.gat_src = d_gsrc_;
         dev_.inv_off = d_inv_off_; dev_.Inv = d_Inv_; dev_.xinv_off = d_xinv_off_; dev_.Xinv = d_Xinv_;
         ensure_dynamic_smem((const void *)mf::k_update<T>, (int)kUpdateSmem);
+        ensure_dynamic_smem((const void *)mf::k_update_next<T>, (int)kUpdateSmem);
+        ensure_dynamic_smem((const void *)mf::k_update_rest<T>, (int)(mf::kRestGroups * kUpdateSmem));
         if constexpr (std::is_same<T, float>::value)
             ensure_dynamic_smem((const void *)mf::k_update_sp, mf::tcu::kSmem);
         ensure_dynamic_smem((const void *)mf::k_panel<T>, (int)kPanelSmem);
@@ -1396,6 +1547,7 @@ public:
             // at once only to the columns of the super-panel (its first 64 columns on the main stream before the
             // next panel, the rest on a second stream overlapping the next panel and its solve); everything right
             // of the super-panel takes the whole super-panel's update in one pass at its end (K = 256)
+            bool bulk_open = false;  // the third stream has an update that the main stream has not waited for
             for (int K0 = 0, sp = 0; K0 < maxc; K0 += mf::tcu::SPW, sp++) {
                 int np = 0, prev_cnt = 0, prev_k0 = 0, prev_p1 = 0;
                 for (int k0 = K0; k0 < std::min(maxc, K0 + mf::tcu::SPW); k0 += mf::PW, np++) {
@@ -1432,10 +1584,26 @@ public:
                 // the last step's first 64 columns lie right of the super-panel: they are part of its update
                 if (np >= 1) cuda_check(cudaStreamWaitEvent(st, rest_ev_[(np - 1) % 2], 0), "cudaStreamWaitEvent");
                 const SpStep &ps = sp_plan_[l][sp];
+                // what lies right of the next super-panel is updated on a third stream, beside that one's chain of panels
+                const int32_t *si = d_sp_.p + ps.si_off, *tnext = si + ps.si_cnt, *trest = tnext + ps.si_cnt + 1;
+                if (ps.si_rest > 0) {
+                    cuda_check(cudaEventRecord(chain_ev_, st), "cudaEventRecord");
+                    cuda_check(cudaStreamWaitEvent(bulk_, chain_ev_, 0), "cudaStreamWaitEvent");
+                }
+                if (bulk_open) cuda_check(cudaStreamWaitEvent(st, bulk_ev_, 0), "cudaStreamWaitEvent");
+                bulk_open = false;
                 if (ps.tc_cnt > 0) launch_tc(ps, K0, st);
-                if (ps.si_cnt > 0)
-                    mf::k_update<T><<<dim3(std::min(ps.si_tiles, std::max(1, 592 / ps.si_cnt)), ps.si_cnt), 256, kUpdateSmem,
-                                      st>>>(dev_, d_sp_.p + ps.si_off, K0, mf::tcu::SPW, 0, 0);
+                if (ps.si_next > 0)
+                    launch_urgent(mf::k_update_next<T>, dim3(ps.si_next), kUpdateSmem, st, dev_, si, tnext, ps.si_cnt, K0,
+                                  (int)mf::tcu::SPW);
+                if (ps.si_rest > 0) {
+                    const int sms = ps.si_next > 0 ? 148 - kChainSms : 148;
+                    const int grid = std::min((ps.si_rest + mf::kRestGroups - 1) / mf::kRestGroups, sms);
+                    mf::k_update_rest<T><<<grid, mf::kRestThreads, mf::kRestGroups * kUpdateSmem, bulk_>>>(dev_, si, trest, ps.si_cnt, K0,
+                                                                                                       mf::tcu::SPW);
+                    cuda_check(cudaEventRecord(bulk_ev_, bulk_), "cudaEventRecord");
+                    bulk_open = true;
+                }
             }
             if (xinv_pass_start_[l + 1] > xinv_pass_start_[l]) {
                 cuda_check(cudaEventRecord(fork_ev_[l], st), "cudaEventRecord");
@@ -1453,6 +1621,7 @@ public:
                 default: mf::k_xinv_reduce<T, 1><<<nt, 256, 0, side_>>>(dev_, tk, d_xinv_w_); break;
                 }
             }
+            if (bulk_open) cuda_check(cudaStreamWaitEvent(st, bulk_ev_, 0), "cudaStreamWaitEvent");
         }
         if (side_used) {
             cuda_check(cudaEventRecord(join_ev_, side_), "cudaEventRecord");
@@ -1532,11 +1701,21 @@ public:
                     int sn = lvl_sorted_[q], region = S.m[sn] - std::min(K0 + SPW, S.ncol[sn]);
                     if (region > 0 && !(use_tc_ && region >= tc_rows_)) {
                         lists.push_back(sn);
-                        int nti = (region + mf::UT - 1) / mf::UT;
-                        ps.si_tiles = std::max(ps.si_tiles, nti * (nti + 1) / 2);
                     }
                 }
                 ps.si_cnt = (int)lists.size() - ps.si_off;
+                for (int next = 1; next >= 0; next--) {
+                    int64_t total = 0;
+                    lists.push_back(0);
+                    for (int i = 0; i < ps.si_cnt; i++) {
+                        int sn = lists[ps.si_off + i], rs = std::min(K0 + SPW, S.ncol[sn]);
+                        int64_t nti = (S.m[sn] - rs + mf::UT - 1) / mf::UT, na = mf::next_tiles(S.ncol[sn], rs, SPW);
+                        total += next ? na * nti - na * (na - 1) / 2 : (nti - na) * (nti - na + 1) / 2;
+                        if (total > INT_MAX) throw Failure(IFEA_INPUT_INVALID, "trailing update larger than one launch");
+                        lists.push_back((int32_t)total);
+                    }
+                    (next ? ps.si_next : ps.si_rest) = (int)total;
+                }
                 sp_plan_[l].push_back(ps);
             }
         }
@@ -1638,14 +1817,17 @@ private:
     DBuf<float4> d_pack_;                       // packed super-panel operands of one level
     cudaStream_t cap_ = nullptr, side_ = nullptr;  // capture stream; side stream of the inverse passes
     cudaStream_t ahead_ = nullptr;                  // look-ahead stream of the trailing updates
+    cudaStream_t bulk_ = nullptr;                   // updates right of the next super-panel
+    cudaEvent_t chain_ev_ = nullptr, bulk_ev_ = nullptr;
     cudaEvent_t trsm_ev_ = nullptr, rest_ev_[2] = {nullptr, nullptr};
     int prio_hi_ = 0;  // greatest stream priority of the device
     std::vector<cudaEvent_t> fork_ev_;
     cudaEvent_t join_ev_ = nullptr;
     cudaGraphExec_t factor_exec_ = nullptr;
     const double *factor_vals_ = nullptr;
+    static constexpr int kChainSms = 20;  // SMs left to a chain of panels beside an update
     static constexpr size_t kUpdateSmem = 2 * mf::PW * mf::SST * sizeof(T);
-    static constexpr size_t kPairSmem = 2 * mf::PW * mf::SST * sizeof(T);
+    static constexpr size_t kPairSmem = std::max(2 * mf::PW * mf::SST, 2 * mf::kPairBuf) * sizeof(T);
     static constexpr size_t kPanelSmem = 2 * mf::PW * (mf::PW + 1) * sizeof(T) + 32 * 33 * sizeof(T);
     cudaStream_t st_;
     cusolverSpHandle_t hsp_ = nullptr;
