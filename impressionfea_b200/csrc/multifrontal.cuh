@@ -147,274 +147,248 @@ static __global__ void k_extend(Dev<T> D, const int32_t *__restrict__ children, 
     }
 }
 
-// Reciprocal of a pivot on the panel's critical path: the fast single-precision intrinsic as the seed, refined by
-// Newton-Raphson steps r <- r (2 - x r), each of which doubles the correct bits (one step for float, two for
-// double); pivots outside the seed's safe range take a plain division.
-__device__ __forceinline__ float recip_rn(float x)
+// Reciprocal of a pivot on the panel's critical path: the hardware's approximate reciprocal r as the seed (20 bits or
+// more), then one third-order step r (1 + e + e^2) with e = 1 - x r (Householder's method; three dependent FMAs), which
+// leaves the rounding of the last one. Only pivots inside panel_range come here: the seed is exact about nothing else.
+__device__ __forceinline__ float panel_recip(float x)
 {
-    if (!(fabsf(x) > 1e-30f && fabsf(x) < 1e30f)) return 1.0f / x;
-    float r = __fdividef(1.0f, x);
-    return r * fmaf(-x, r, 2.0f);
+    const float r = __fdividef(1.0f, x), e = fmaf(-x, r, 1.0f);
+    return fmaf(r, fmaf(e, e, e), r);
 }
-__device__ __forceinline__ double recip_rn(double x)
+__device__ __forceinline__ double panel_recip(double x)
 {
-    if (!(fabs(x) > 1e-30 && fabs(x) < 1e30)) return 1.0 / x;
-    double r = (double)__fdividef(1.0f, (float)x);
-    r = r * fma(-x, r, 2.0);
-    return r * fma(-x, r, 2.0);
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
 }
+__device__ __forceinline__ bool panel_range(float x) { return x > 1e-30f && x < 1e30f; }
+__device__ __forceinline__ bool panel_range(double x) { return x > 1e-290 && x < 1e290; }
 
-// Recursive-doubling merge of the panel inverse at block size H: for every pair of H x H diagonal blocks,
-// X21 = -X22 (L21 X11). The upper triangles of X11 and X22 are zero, so the dot products run over whole blocks.
-template <typename T, int H>
-__device__ __forceinline__ void panel_merge(T (*Ds)[PW + 1], T (*Xs)[PW + 1], T (*Ts)[33], int tid)
+// L D L^T of an 8 x 8 block (lower triangle, in registers): B becomes L D below the diagonal and D on it, rd = 1 / D.
+// The chain from pivot to pivot is a reciprocal, a product and an FMA.
+template <bool SAFE, typename T>
+__device__ __forceinline__ void panel_factor8(T (&B)[8][8], T (&L)[8][8], T (&rd)[8])
 {
-    constexpr int PER = H * H, TOTAL = (PW / (2 * H)) * PER, PT = TOTAL / 256;  // entries per thread: 1, 2, 4
-    T v[PT];
-#pragma unroll
-    for (int k = 0; k < PT; k++) {
-        int t = tid + 256 * k, p = t / PER, e = t % PER, i = e / H, j = e % H, b = p * 2 * H;
-        T a0 = 0, a1 = 0;
-#pragma unroll
-        for (int q = 0; q < H; q += 2) {
-            a0 = fma(Ds[b + H + i][b + q], Xs[b + q][b + j], a0);
-            a1 = fma(Ds[b + H + i][b + q + 1], Xs[b + q + 1][b + j], a1);
-        }
-        v[k] = a0 + a1;
-    }
-#pragma unroll
-    for (int k = 0; k < PT; k++) {
-        int t = tid + 256 * k, p = t / PER, e = t % PER, i = e / H, j = e % H;
-        Ts[p * H + i][j] = v[k];  // the pairs of one size fill 32 rows
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < PT; k++) {
-        int t = tid + 256 * k, p = t / PER, e = t % PER, i = e / H, j = e % H, b = p * 2 * H;
-        T a0 = 0, a1 = 0;
-#pragma unroll
-        for (int q = 0; q < H; q += 2) {
-            a0 = fma(Xs[b + H + i][b + H + q], Ts[p * H + q][j], a0);
-            a1 = fma(Xs[b + H + i][b + H + q + 1], Ts[p * H + q + 1][j], a1);
-        }
-        v[k] = a0 + a1;
-    }
-#pragma unroll
-    for (int k = 0; k < PT; k++) {
-        int t = tid + 256 * k, p = t / PER, e = t % PER, i = e / H, j = e % H, b = p * 2 * H;
-        Xs[b + H + i][b + j] = -v[k];
-    }
-    __syncthreads();
-}
-
-// Warp-level L D L^T of the eight columns J .. J + 7 of the panel block over rows J .. 63. Every lane factors the
-// 8 x 8 diagonal block in registers (no shuffles on the pivot chain), then eliminates its own rows J + 8 + lane and
-// J + 40 + lane against it. Reciprocal pivots go to rdv, the lowest failing column to *fail.
-template <typename T>
-__device__ __forceinline__ void panel_factor8(T (*Ds)[PW + 1], T *rdv, int *fail, int J, int lane)
-{
-    T B[8][8], L[8][8], rd[8];
-#pragma unroll
-    for (int i = 0; i < 8; i++)
-#pragma unroll
-        for (int j = 0; j <= i; j++) B[i][j] = Ds[J + i][J + j];
-    int bad = -1;
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        if (!(B[k][k] > 0) && bad < 0) bad = k;
-        rd[k] = recip_rn(B[k][k]);
+        rd[k] = SAFE ? T(1) / B[k][k] : panel_recip(B[k][k]);
 #pragma unroll
         for (int i = k + 1; i < 8; i++) {
             L[i][k] = B[i][k] * rd[k];
+            B[i][i] = fma(-L[i][k], B[i][k], B[i][i]);
 #pragma unroll
-            for (int j = k + 1; j <= i; j++) B[i][j] = fma(-L[i][k], B[j][k], B[i][j]);
+            for (int j = k + 1; j < i; j++) B[i][j] = fma(-L[i][k], B[j][k], B[i][j]);
         }
     }
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        int r = J + 8 + lane + 32 * h;
-        if (r >= PW) continue;
-        T u[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            T v = Ds[r][J + k];
-#pragma unroll
-            for (int j = 0; j < k; j++) v = fma(-u[j], L[k][j], v);
-            u[k] = v;
-        }
-#pragma unroll
-        for (int k = 0; k < 8; k++) Ds[r][J + k] = u[k];
+}
+
+// acc += A B of an 8 x 8 tile by a warp, entries (lane / 4, 2 (lane % 4) + e): A(r, k) = A[r * lda + k],
+// B(k, c) = B[k * ldk + c * ldc], K a multiple of eight. Two sums, of alternate fours in k.
+__device__ __forceinline__ void tile8(const double *A, int lda, const double *B, int ldk, int ldc, int K, int lane, double (&acc)[2])
+{
+    double s0[2] = {0, 0}, s1[2] = {0, 0};
+    const int r = lane >> 2, q = lane & 3;
+    for (int k = 0; k < K; k += 8) {
+        const double a0 = A[r * lda + k + q], b0 = B[(k + q) * ldk + r * ldc], a1 = A[r * lda + k + 4 + q], b1 = B[(k + 4 + q) * ldk + r * ldc];
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(s0[0]), "+d"(s0[1]) : "d"(a0), "d"(b0));
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(s1[0]), "+d"(s1[1]) : "d"(a1), "d"(b1));
     }
-    __syncwarp();  // every lane has read the diagonal block
-    if (lane == 0) {
+    acc[0] = s0[0] + s1[0], acc[1] = s0[1] + s1[1];
+}
+__device__ __forceinline__ void tile8(const float *A, int lda, const float *B, int ldk, int ldc, int K, int lane, float (&acc)[2])
+{
+    float s0[2] = {0, 0}, s1[2] = {0, 0};
+    const int r = lane >> 2, c = 2 * (lane & 3);
+    for (int k = 0; k < K; k += 8)
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
+        for (int j = 0; j < 4; j++) {
+            const float a0 = A[r * lda + k + j], a1 = A[r * lda + k + 4 + j];
 #pragma unroll
-            for (int j = 0; j <= i; j++) Ds[J + i][J + j] = B[i][j];
-            rdv[J + i] = rd[i];
+            for (int e = 0; e < 2; e++) {
+                s0[e] = fmaf(a0, B[(k + j) * ldk + (c + e) * ldc], s0[e]);
+                s1[e] = fmaf(a1, B[(k + 4 + j) * ldk + (c + e) * ldc], s1[e]);
+            }
         }
+    acc[0] = s0[0] + s1[0], acc[1] = s0[1] + s1[1];
+}
+
+constexpr int PST = PW + 2, PLT = 9;  // row strides of the panel's blocks in shared memory
+
+// Recursive-doubling merge of the inverse X of the block's Cholesky factor L at block size H, by eight warps: for every
+// pair of H x H diagonal blocks X21 = -X22 (L21 X11), in 8 x 8 tiles, the inner product in the unused upper right
+// block. Tiles right of the diagonal ones of X11 and X22 are zero and are not read.
+template <int H, typename T>
+__device__ __forceinline__ void panel_merge(const T *Ls, T *Xs, int warp, int lane)
+{
+    constexpr int G = H / 8, NT = PW / (2 * H) * G * G;  // 4, 8, 16 tiles
+    const int r = lane >> 2, c = 2 * (lane & 3);
+#pragma unroll
+    for (int pass = 0; pass < 2; pass++) {
+#pragma unroll
+        for (int q = 0; q < (NT + 7) / 8; q++) {
+            const int t = warp + 8 * q;
+            if (t >= NT) break;
+            const int base = t / (G * G) * 2 * H, i = t / G % G, j = q == 0 ? t % G : G - 1 - t % G;  // (long ones with short ones)
+            T acc[2];
+            if (pass == 0)
+                tile8(Ls + (base + H + 8 * i) * PST + base + 8 * j, PST, Xs + (base + 8 * j) * PST + base + 8 * j, PST, 1, H - 8 * j, lane, acc);
+            else
+                tile8(Xs + (base + H + 8 * i) * PST + base + H, PST, Xs + base * PST + base + H + 8 * j, PST, 1, 8 * i + 8, lane, acc);
+            T *o = pass == 0 ? Xs + (base + 8 * i + r) * PST + base + H + 8 * j + c : Xs + (base + H + 8 * i + r) * PST + base + 8 * j + c;
+            o[0] = pass == 0 ? acc[0] : -acc[0], o[1] = pass == 0 ? acc[1] : -acc[1];
+        }
+        __syncthreads();
     }
-    if (lane == 0 && bad >= 0) *fail = J + bad;
 }
 
 // Panel k0 of every listed front: Cholesky of the diagonal block and the block's inverse (kept for the rows below
-// and for the solves). Blocked L D L^T in shared memory: warp 0 factors eight columns at a time over all rows
-// below them (in registers, no block barrier) while the other warps apply the previous eight to the columns beyond
-// them; the pivot columns are scaled to Cholesky form at the end. Rows and columns at or beyond the block width
-// are the identity. The inverse is built by recursive doubling: the 8x8 diagonal blocks by forward substitution in
-// registers, then merges at sizes 8, 16 and 32. The lowest failing pivot column (new numbering) goes to err.
-// Dynamic shared memory: two 64 x 65 blocks and a 32 x 33 one.
+// and for the solves), as a blocked L D L^T in shared memory, eight columns at a time:
+//   - warps 0 and 1 factor the 8 x 8 block, every lane in registers, and each lane takes its row through it; the other
+//     warps wait (work on the inverse or the stores beside them made these two 2 to 3 times as slow);
+//   - then all warps update the columns to the right, in 8 x 8 tiles.
+// The inverse is built by recursive doubling: the 8 x 8 diagonal blocks by substitution, then merges at 8, 16 and 32.
+// What bounds a panel is this chain: B200, FP64, 64 columns: 13.1 us (2,000 cycles for eight columns, of which the
+// pivots take 460; 4,000 until the block is loaded). With one warp for the rows, which took 2,500 cycles, and the
+// merges without the tensor cores it took 19.5.
+// Rows and columns at or beyond the block width are the identity. The lowest failing pivot column (new numbering) goes
+// to err. Dynamic shared memory: two 64 x 66 blocks and a 64 x 9 one.
 template <typename T>
 static __global__ void __launch_bounds__(256) k_panel(Dev<T> D, const int32_t *__restrict__ fronts, int k0, int *err)
 {
     extern __shared__ __align__(16) unsigned char shp_raw[];
-    T *shp = (T *)shp_raw;
-    T (*Ds)[PW + 1] = (T (*)[PW + 1])shp;
-    T (*Xs)[PW + 1] = (T (*)[PW + 1])(shp + PW * (PW + 1));
-    T (*Ts)[33] = (T (*)[33])(shp + 2 * PW * (PW + 1));
-    __shared__ T rdv[PW];  // reciprocal pivots, then the square roots of the pivots
-    __shared__ T rsq[PW];  // reciprocal square roots of the pivots
+    T *Ls = (T *)shp_raw;      // L D below the diagonal, D on it; at the end the Cholesky factor
+    T *Xs = Ls + PW * PST;     // the inverse
+    T *Lt = Xs + PW * PST;     // L of the current eight columns
+    __shared__ T sq[PW], rs[PW];  // roots of the pivots and their reciprocals
     __shared__ int fail;
-    int s = fronts[blockIdx.x];
-    int ms = D.m[s], w = min(PW, D.ncol[s] - k0);
-    T *F = D.F + D.front_off[s];
+    __shared__ unsigned char tiles[28];  // the lower triangle's tiles row by row: row << 4 | column
+    const int s = fronts[blockIdx.x], tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ms = D.m[s], w = min(PW, D.ncol[s] - k0);
+    T *F = D.F + D.front_off[s] + (int64_t)k0 * ms + k0;
     T *Inv = D.Inv + D.inv_off[s] + (int64_t)(k0 / PW) * PW * PW;
-    int tid = threadIdx.x, lane = tid & 31, r = tid & (PW - 1), cg = tid >> 6;
     {
         T v[16];  // all sixteen loads of a thread in flight before any store
 #pragma unroll
         for (int i = 0; i < 16; i++) {
             int t = tid + 256 * i, rr = t % PW, c = t / PW;
             v[i] = rr == c ? T(1) : T(0);
-            if (rr < w && c < w && rr >= c) v[i] = F[(int64_t)(k0 + c) * ms + k0 + rr];
+            if (rr < w && c < w && rr >= c) v[i] = F[(int64_t)c * ms + rr];
         }
 #pragma unroll
         for (int i = 0; i < 16; i++) {
-            int t = tid + 256 * i, rr = t % PW, c = t / PW;
-            Ds[rr][c] = v[i];
-            Xs[rr][c] = T(0);
+            int t = tid + 256 * i;
+            Ls[(t % PW) * PST + t / PW] = v[i];
         }
     }
     if (tid == 0) fail = -1;
+    if (tid < 28) {
+        int tr = 0, tc = tid;
+        while (tc > tr) tc -= ++tr;
+        tiles[tid] = (unsigned char)(tr << 4 | tc);
+    }
     __syncthreads();
-    if (tid < 32) panel_factor8(Ds, rdv, &fail, 0, lane);
-    __syncthreads();
-    // look-ahead inside the block: the CTA applies block J to the next eight columns, then warp 0 factors them
-    // while the other warps apply block J to the columns beyond; two barriers per eight columns
-    for (int J = 0; J < PW; J += 8) {
+    for (int J = 0; J < w; J += 8) {
+        const int r = J + tid;  // a lane's row; the first eight are the block's own
+        T u[8];
+        if (warp < 2) {
+            T B[8][8], L[8][8], rd[8];
+            auto load = [&]() {
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+#pragma unroll
+                    for (int j = 0; j <= i; j++) B[i][j] = Ls[(J + i) * PST + J + j];
+            };
+            load();
+#pragma unroll
+            for (int k = 0; k < 8; k++) u[k] = r < PW ? Ls[r * PST + J + k] : T(0);
+            panel_factor8<false>(B, L, rd);
+            bool in = true;
+#pragma unroll
+            for (int k = 0; k < 8; k++) in = in && panel_range(B[k][k]);
+            if (!in) {  // (every lane of both warps holds the same block)
+                load();
+                panel_factor8<true>(B, L, rd);
+                int bad = -1;
+#pragma unroll
+                for (int k = 7; k >= 0; k--)
+                    if (!(B[k][k] > 0)) bad = k;
+                if (tid == 0 && bad >= 0) fail = J + bad;
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+#pragma unroll
+                for (int j = k + 1; j < 8; j++) u[j] = fma(-u[k], L[j][k], u[j]);
+                if (tid >= 8 && r < PW) {
+                    Ls[r * PST + J + k] = u[k];
+                    Lt[r * PLT + k] = u[k] * rd[k];
+                }
+            }
+        }
+        __syncthreads();
         if (fail >= 0) {
             if (tid == 0) atomicMin(err, D.c0[s] + k0 + fail);
             return;  // every thread read the same flag: a uniform exit
         }
-        if (J + 8 < PW) {
-            // the next eight columns (rows J + 8 .. 63) with block J, spread over the whole CTA
-            T v[2];
+        if (tid < 8)  // (both warps have read the block)
 #pragma unroll
-            for (int i = 0; i < 2; i++) {  // 8 x 56 entries at most: two per thread, loads before stores
-                int e = tid + 256 * i, c = J + 8 + (e & 7), rr = J + 8 + (e >> 3);
-                v[i] = T(0);
-                if (rr >= PW || c > rr) continue;
-                T v0 = Ds[rr][c], v1 = T(0);
+            for (int k = 0; k < 8; k++)
+                if (k <= tid) Ls[r * PST + J + k] = u[k];
+        const int ntile = (PW - 8 - J) / 8 * ((PW - J) / 8) / 2;
+        T acc[4][2];
 #pragma unroll
-                for (int q = 0; q < 8; q += 2) {
-                    v0 = fma(-Ds[rr][J + q] * rdv[J + q], Ds[c][J + q], v0);
-                    v1 = fma(-Ds[rr][J + q + 1] * rdv[J + q + 1], Ds[c][J + q + 1], v1);
-                }
-                v[i] = v0 + v1;
+        for (int i = 0; i < 4; i++) {
+            if (7 - warp + 8 * i < ntile) {
+                const int rc = tiles[7 - warp + 8 * i], r0 = J + 8 + 8 * (rc >> 4), c0 = J + 8 + 8 * (rc & 15);
+                tile8(Ls + r0 * PST + J, PST, Lt + c0 * PLT, 1, PLT, 8, lane, acc[i]);
             }
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                int e = tid + 256 * i, c = J + 8 + (e & 7), rr = J + 8 + (e >> 3);
-                if (rr < PW && c <= rr) Ds[rr][c] = v[i];
-            }
-            __syncthreads();
         }
-        if (tid < 32) {
-            if (J + 8 < PW) panel_factor8(Ds, rdv, &fail, J + 8, lane);
-        } else {
-            // columns (and rows) J + 16 .. 63: thread u keeps row J + 16 + u % 56 and walks every fourth column
-            int u = tid - 32, rr = J + 16 + u % 56, c0 = J + 16 + u / 56;
-            if (rr < PW) {
-                T lr[8], v[12];
 #pragma unroll
-                for (int q = 0; q < 8; q++) lr[q] = Ds[rr][J + q] * rdv[J + q];
-                // all loads first (at most twelve columns per thread), then the stores
-#pragma unroll
-                for (int i = 0; i < 12; i++) {
-                    int c = c0 + 4 * i;
-                    if (c > rr) break;
-                    T v0 = Ds[rr][c], v1 = T(0);
-#pragma unroll
-                    for (int q = 0; q < 8; q += 2) {
-                        v0 = fma(-lr[q], Ds[c][J + q], v0);
-                        v1 = fma(-lr[q + 1], Ds[c][J + q + 1], v1);
-                    }
-                    v[i] = v0 + v1;
-                }
-#pragma unroll
-                for (int i = 0; i < 12; i++) {
-                    int c = c0 + 4 * i;
-                    if (c > rr) break;
-                    Ds[rr][c] = v[i];
-                }
+        for (int i = 0; i < 4; i++) {
+            if (7 - warp + 8 * i < ntile) {
+                const int rc = tiles[7 - warp + 8 * i], r0 = J + 8 + 8 * (rc >> 4), c0 = J + 8 + 8 * (rc & 15);
+                T *o = Ls + (r0 + (lane >> 2)) * PST + c0 + 2 * (lane & 3);
+                o[0] -= acc[i][0], o[1] -= acc[i][1];
             }
         }
         __syncthreads();
     }
     if (tid < PW) {
-        T q = sqrt(Ds[tid][tid]);
-        rdv[tid] = q;
-        rsq[tid] = T(1) / q;
+        const T q = sqrt(Ls[tid * PST + tid]);
+        sq[tid] = q;
+        rs[tid] = T(1) / q;
     }
     __syncthreads();
-    {
-        T v[16];
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            int c = cg + 4 * i;
-            v[i] = c == r ? rdv[r] : c < r ? Ds[r][c] * rsq[c] : T(0);
-        }
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            int c = cg + 4 * i;
-            if (c <= r) Ds[r][c] = v[i];
-        }
+    for (int i = 0; i < 16; i++) {
+        const int t = tid + 256 * i, rr = t % PW, c = t / PW;
+        if (rr < c) continue;
+        const T v = rr == c ? sq[c] : Ls[rr * PST + c] * rs[c];
+        Ls[rr * PST + c] = v;
+        if (rr < w && c < w) F[(int64_t)c * ms + rr] = v;
     }
     __syncthreads();
-    {
-        T v[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            int t = tid + 256 * i;
-            v[i] = Ds[t % PW][t / PW];
-        }
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            int t = tid + 256 * i, rr = t % PW, c = t / PW;
-            if (rr < w && c < w && rr >= c) F[(int64_t)(k0 + c) * ms + k0 + rr] = v[i];
-        }
-    }
-    // 8x8 diagonal blocks: thread (b, j) forward-substitutes column j of block b
-    if (tid < PW) {
-        int b8 = (tid >> 3) * 8, j = tid & 7;
+    if (tid < PW) {  // 8 x 8 diagonal blocks: thread (b, j) substitutes for column j of block b
+        const int b = tid & ~7, j = tid & 7;
         T x[8];
 #pragma unroll
+        for (int i = 0; i < 8; i++) x[i] = i == j ? T(1) : T(0);
+#pragma unroll
         for (int i = 0; i < 8; i++) {
-            T v = i == j ? T(1) : T(0);
+            x[i] *= rs[b + i];
+            Xs[(b + i) * PST + b + j] = x[i];
 #pragma unroll
-            for (int q = 0; q < i; q++) v = fma(-Ds[b8 + i][b8 + q], x[q], v);
-            x[i] = v * rsq[b8 + i];  // 1 / L_ii
+            for (int k = i + 1; k < 8; k++) x[k] = fma(-Ls[(b + k) * PST + b + i], x[i], x[k]);
         }
-#pragma unroll
-        for (int i = 0; i < 8; i++) Xs[b8 + i][b8 + j] = x[i];
     }
     __syncthreads();
-    panel_merge<T, 8>(Ds, Xs, Ts, tid);
-    panel_merge<T, 16>(Ds, Xs, Ts, tid);
-    panel_merge<T, 32>(Ds, Xs, Ts, tid);
-    for (int t = tid; t < PW * PW; t += blockDim.x) {
-        int i = t % PW, c = t / PW;
-        Inv[t] = (i < w && c < w) ? Xs[i][c] : T(0);  // column-major, row i
+    panel_merge<8>(Ls, Xs, warp, lane);
+    panel_merge<16>(Ls, Xs, warp, lane);
+    panel_merge<32>(Ls, Xs, warp, lane);
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const int t = tid + 256 * i, rr = t % PW, c = t / PW;
+        Inv[t] = rr < w && c < w && rr >= c ? Xs[rr * PST + c] : T(0);  // column-major
     }
 }
 
@@ -1828,7 +1802,7 @@ private:
     static constexpr int kChainSms = 20;  // SMs left to a chain of panels beside an update
     static constexpr size_t kUpdateSmem = 2 * mf::PW * mf::SST * sizeof(T);
     static constexpr size_t kPairSmem = std::max(2 * mf::PW * mf::SST, 2 * mf::kPairBuf) * sizeof(T);
-    static constexpr size_t kPanelSmem = 2 * mf::PW * (mf::PW + 1) * sizeof(T) + 32 * 33 * sizeof(T);
+    static constexpr size_t kPanelSmem = (2 * mf::PW * mf::PST + mf::PW * mf::PLT) * sizeof(T);
     cudaStream_t st_;
     cusolverSpHandle_t hsp_ = nullptr;
     std::vector<int64_t> inv_off_, xinv_off_;
