@@ -363,6 +363,8 @@ struct Forging3D {
     HostPinned<int32_t> hi;
     int wpb = 8;          // warps per block of the column kernels
     size_t col_smem = 0;  // dynamic shared memory of the column kernels
+    int max_ring = 1;     // most nodes around one, itself among them
+    int ring_warps() const { return std::max(1, std::min(8, 160 * 1024 / (24 * max_ring))); }
 
     Forging3D(const ifea3d_params &p) : P(p)
     {
@@ -654,7 +656,8 @@ struct Forging3D {
         d_elrate.zero(st);
         // column-kernel launch shape: chunk of 9*max_nbr doubles per warp in shared memory
         size_t per_warp = 9 * (size_t)topo.max_nbr * sizeof(double);
-        wpb = (int)std::max<size_t>(1, std::min<size_t>(8, (160 * 1024) / std::max<size_t>(per_warp, 1)));
+        // (two blocks an SM where ten warps' chunks, or fewer, leave room for them)
+        wpb = (int)std::max<size_t>(1, std::min<size_t>(kColumnWarps, (112 * 1024) / std::max<size_t>(per_warp, 1)));
         col_smem = per_warp * wpb;
         if (per_warp > 200 * 1024) throw Failure(IFEA_INPUT_INVALID, "node neighbourhood too large for the column kernel");
         auto set_smem = [&](const void *f) {
@@ -665,6 +668,9 @@ struct Forging3D {
         set_smem((const void *)k_columns<ASM_RESIDUAL, false>);
         set_smem((const void *)k_columns<ASM_ENERGY, false>);
         set_smem((const void *)k_kvol);
+        max_ring = 1;
+        for (int n = 0; n < topo.nn; n++) max_ring = std::max(max_ring, topo.g_start[n + 1] - topo.g_start[n]);
+        ensure_dynamic_smem((const void *)k_anp_coef, ring_warps() * 3 * max_ring * (int)sizeof(double));
         need_analyze = true;
         have_factor = false;
         pcg_failures = pcg_skip = 0;
@@ -783,7 +789,8 @@ struct Forging3D {
         int32_t e4[4];
         read_err(e4);
         if (e4[0] != INT_MAX) throw Failure(IFEA_MESH_DISTORTED, fmt("Tetrahedron %d is inverted at step %d.", e4[0], step_index));
-        k_anp_coef<<<grid(topo.nn), 256, 0, st>>>(V);
+        const int rw = ring_warps();
+        k_anp_coef<<<std::min(8 * 148, (topo.nn + rw - 1) / rw), rw * 32, rw * 3 * max_ring * sizeof(double), st>>>(V, max_ring);
         int G = (int)topo.g_node.size();
         k_clocal<<<grid(G), 256, 0, st>>>(V, G);
         k_kvol<<<std::min(kReduceBlocks * 2, (topo.nn + wpb - 1) / wpb), wpb * 32, col_smem, st>>>(V, topo.max_nbr);
