@@ -636,7 +636,7 @@ def run_gpu(args, rank, world):
                              "frac": f_ach / tflops_peak if f_ach else None, "peak_kind": peak_kind + " (bf16 dense, sustained)",
                              "traffic": None, "gflop_per_launch": gflop, "ms_per_launch": factor_ms,
                              "launches": int(nf)},
-                "roofline_solve": {"kernel": "multifrontal triangular-solve sweep (forward + backward, one graph)",
+                "roofline_solve": {"kernel": "multifrontal triangular-solve sweep (forward + backward, one persistent kernel)",
                                    "bound": "hbm", "achieved": s_ach, "peak": hbm_peak, "unit": "GB/s",
                                    "frac": s_ach / hbm_peak if s_ach else None, "algorithmic_bytes": sbytes,
                                    "ms_per_launch": solve_ms, "launches": int(n_solves)},
