@@ -1,14 +1,91 @@
 // spd_capi.cu — C ABI of the GPU sparse SPD solver (ifea_spd_*), shaped like the reference's ISpdSolver
 // (Solver/Linear/ISpdSolver.cs:24-41) so a CudssSolver-style P/Invoke backend can bind it directly.
+#include <algorithm>
+#include <cstring>
+#include <exception>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "multifrontal.cuh"
+
+// Uploads a large pageable array: threads copy chunks into pinned slots of their own (two each) and send them on, so
+// that the copies into pinned memory and over the bus overlap. 78 MB take about 2.8 ms
+// (B200, 16 host cores), 7.2 by the driver's own staging of a pageable copy. Below kLeast starting threads takes a good
+// part of what it gains (8 MB: 0.7 ms), and memory that is pinned already is copied directly.
+class HostUpload {
+public:
+    static constexpr size_t kLeast = 8 << 20;
+    ~HostUpload() { release(); }
+    void prepare()
+    {
+        if (buf_) return;
+        ifea::cuda_check(cudaMallocHost((void **)&buf_, kSlots * kChunk), "cudaMallocHost");
+        for (auto &e : ev_) ifea::cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+    }
+    void release()
+    {
+        for (auto &e : ev_) {
+            if (e) cudaEventDestroy(e);
+            e = nullptr;
+        }
+        if (buf_) cudaFreeHost(buf_);
+        buf_ = nullptr;
+    }
+    // src may change once this returns
+    void run(void *dst, const void *src, size_t bytes, cudaStream_t st)
+    {
+        cudaPointerAttributes at{};
+        const bool pageable = cudaPointerGetAttributes(&at, src) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+        if (!pageable) cudaGetLastError();
+        if (!buf_ || bytes < kLeast || !pageable) {
+            ifea::cuda_check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync H2D");
+            return;
+        }
+        int dev = 0;
+        ifea::cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+        cudaError_t err[kThreads] = {};
+        auto work = [&](int t) {
+            cudaError_t e = cudaSetDevice(dev);
+            int k = 0;
+            for (size_t o = t * kChunk; o < bytes && e == cudaSuccess; o += kThreads * kChunk, k++) {
+                const int slot = 2 * t + (k & 1);
+                const size_t n = std::min(kChunk, bytes - o);
+                e = cudaEventSynchronize(ev_[slot]);
+                if (e != cudaSuccess) break;
+                std::memcpy(buf_ + slot * kChunk, (const char *)src + o, n);
+                e = cudaMemcpyAsync((char *)dst + o, buf_ + slot * kChunk, n, cudaMemcpyHostToDevice, st);
+                if (e == cudaSuccess) e = cudaEventRecord(ev_[slot], st);
+            }
+            err[t] = e;
+        };
+        std::thread th[kThreads];
+        for (int t = 1; t < kThreads; t++) {
+            try {
+                th[t] = std::thread(work, t);
+            } catch (const std::exception &) {  // (no thread to be had: its chunks below)
+            }
+        }
+        work(0);
+        for (int t = 1; t < kThreads; t++) {
+            if (th[t].joinable()) th[t].join();
+            else work(t);
+        }
+        for (cudaError_t e : err) ifea::cuda_check(e, "staged upload");
+    }
+
+private:
+    static constexpr int kThreads = 4, kSlots = 2 * kThreads;
+    static constexpr size_t kChunk = 1 << 20;
+    char *buf_ = nullptr;
+    cudaEvent_t ev_[kSlots] = {};
+};
 
 struct ifea_spd {
     cudaStream_t st = nullptr;
     ifea::MfSolver *s = nullptr;
     ifea::DBuf<double> vals, b, x;
+    HostUpload up;
     std::vector<int32_t> col_ptr;
     int n = 0;
     int64_t nnz = 0;
@@ -62,6 +139,7 @@ void ifea_spd_destroy(ifea_spd *h)
     h->vals.release();
     h->b.release();
     h->x.release();
+    h->up.release();
     if (h->st) cudaStreamDestroy(h->st);
     delete h;
 }
@@ -81,6 +159,7 @@ ifea_status ifea_spd_analyze(ifea_spd *h, int32_t n, const int32_t *col_ptr, con
         s.vals.resize(s.nnz);
         s.b.resize(n);
         s.x.resize(n);
+        if (sizeof(double) * (size_t)s.nnz >= HostUpload::kLeast) s.up.prepare();
     });
 }
 
@@ -90,7 +169,7 @@ ifea_status ifea_spd_factorize(ifea_spd *h, const double *values)
     if (!values) return IFEA_INPUT_INVALID;
     return spd_guard(h, [&](ifea_spd &s) {
         if (!s.s->analyzed()) throw ifea::Failure(IFEA_BAD_STATE, "Analyze must be called first.");
-        s.vals.upload(values, s.nnz, s.st);
+        s.up.run(s.vals, values, sizeof(double) * (size_t)s.nnz, s.st);
         s.s->factorize(s.vals);
     });
 }
