@@ -20,8 +20,11 @@ public:
     void prepare()
     {
         if (buf_) return;
-        ifea::cuda_check(cudaMallocHost((void **)&buf_, kSlots * kChunk), "cudaMallocHost");
-        for (auto &e : ev_) ifea::cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+        bool ok = cudaMallocHost((void **)&buf_, kSlots * kChunk) == cudaSuccess;
+        for (auto &e : ev_) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+        if (ok) return;
+        cudaGetLastError();  // (no slots to be had: arrays go up as pageable copies)
+        release();
     }
     void release()
     {
