@@ -717,7 +717,7 @@ static __global__ void __launch_bounds__(256, 3) k_update(Dev<T> D, const int32_
 // 256 threads with a tile each) and the host launches them on fewer SMs than there are.
 // The 57k-equation FP64 factor (B200): one launch over the whole region, 65 CTAs a front whatever its size, four CTAs an
 // SM where three fit and the next panels after it, factorised in 38 ms; tiles in one sequence 32 ms; beside the chain
-// 27.7 ms. Three tiles at work on an SM reach 18 TFLOP/s on 128 SMs (57% of the pipe's rate while an SM works).
+// 27.7 ms, with shorter panels 26.9. Three tiles at work on an SM reach 18 TFLOP/s on 128 SMs (57% of the pipe's rate while an SM works).
 // next_tiles: column tiles of a front's next super-panel, none once its pivot columns are done.
 constexpr int kRestGroups = 3, kRestThreads = 256 * kRestGroups;
 __host__ __device__ inline int next_tiles(int ncol, int rs, int depth)
