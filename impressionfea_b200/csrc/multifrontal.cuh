@@ -150,11 +150,6 @@ static __global__ void k_extend(Dev<T> D, const int32_t *__restrict__ children, 
 // Reciprocal of a pivot on the panel's critical path: the hardware's approximate reciprocal r as the seed (20 bits or
 // more), then one third-order step r (1 + e + e^2) with e = 1 - x r (Householder's method; three dependent FMAs), which
 // leaves the rounding of the last one. Only pivots inside panel_range come here: the seed is exact about nothing else.
-__device__ __forceinline__ float panel_recip(float x)
-{
-    const float r = __fdividef(1.0f, x), e = fmaf(-x, r, 1.0f);
-    return fmaf(r, fmaf(e, e, e), r);
-}
 __device__ __forceinline__ double panel_recip(double x)
 {
     double r;
@@ -162,17 +157,16 @@ __device__ __forceinline__ double panel_recip(double x)
     const double e = fma(-x, r, 1.0);
     return fma(r, fma(e, e, e), r);
 }
-__device__ __forceinline__ bool panel_range(float x) { return x > 1e-30f && x < 1e30f; }
 __device__ __forceinline__ bool panel_range(double x) { return x > 1e-290 && x < 1e290; }
 
 // L D L^T of an 8 x 8 block (lower triangle, in registers): B becomes L D below the diagonal and D on it, rd = 1 / D.
 // The chain from pivot to pivot is a reciprocal, a product and an FMA.
-template <bool SAFE, typename T>
-__device__ __forceinline__ void panel_factor8(T (&B)[8][8], T (&L)[8][8], T (&rd)[8])
+template <bool SAFE>
+__device__ __forceinline__ void panel_factor8(double (&B)[8][8], double (&L)[8][8], double (&rd)[8])
 {
 #pragma unroll
     for (int k = 0; k < 8; k++) {
-        rd[k] = SAFE ? T(1) / B[k][k] : panel_recip(B[k][k]);
+        rd[k] = SAFE ? 1.0 / B[k][k] : panel_recip(B[k][k]);
 #pragma unroll
         for (int i = k + 1; i < 8; i++) {
             L[i][k] = B[i][k] * rd[k];
@@ -196,30 +190,14 @@ __device__ __forceinline__ void tile8(const double *A, int lda, const double *B,
     }
     acc[0] = s0[0] + s1[0], acc[1] = s0[1] + s1[1];
 }
-__device__ __forceinline__ void tile8(const float *A, int lda, const float *B, int ldk, int ldc, int K, int lane, float (&acc)[2])
-{
-    float s0[2] = {0, 0}, s1[2] = {0, 0};
-    const int r = lane >> 2, c = 2 * (lane & 3);
-    for (int k = 0; k < K; k += 8)
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const float a0 = A[r * lda + k + j], a1 = A[r * lda + k + 4 + j];
-#pragma unroll
-            for (int e = 0; e < 2; e++) {
-                s0[e] = fmaf(a0, B[(k + j) * ldk + (c + e) * ldc], s0[e]);
-                s1[e] = fmaf(a1, B[(k + 4 + j) * ldk + (c + e) * ldc], s1[e]);
-            }
-        }
-    acc[0] = s0[0] + s1[0], acc[1] = s0[1] + s1[1];
-}
 
 constexpr int PST = PW + 2, PLT = 9;  // row strides of the panel's blocks in shared memory
 
 // Recursive-doubling merge of the inverse X of the block's Cholesky factor L at block size H, by eight warps: for every
 // pair of H x H diagonal blocks X21 = -X22 (L21 X11), in 8 x 8 tiles, the inner product in the unused upper right
 // block. Tiles right of the diagonal ones of X11 and X22 are zero and are not read.
-template <int H, typename T>
-__device__ __forceinline__ void panel_merge(const T *Ls, T *Xs, int warp, int lane)
+template <int H>
+__device__ __forceinline__ void panel_merge(const double *Ls, double *Xs, int warp, int lane)
 {
     constexpr int G = H / 8, NT = PW / (2 * H) * G * G;  // 4, 8, 16 tiles
     const int r = lane >> 2, c = 2 * (lane & 3);
@@ -230,12 +208,12 @@ __device__ __forceinline__ void panel_merge(const T *Ls, T *Xs, int warp, int la
             const int t = warp + 8 * q;
             if (t >= NT) break;
             const int base = t / (G * G) * 2 * H, i = t / G % G, j = q == 0 ? t % G : G - 1 - t % G;  // (long ones with short ones)
-            T acc[2];
+            double acc[2];
             if (pass == 0)
                 tile8(Ls + (base + H + 8 * i) * PST + base + 8 * j, PST, Xs + (base + 8 * j) * PST + base + 8 * j, PST, 1, H - 8 * j, lane, acc);
             else
                 tile8(Xs + (base + H + 8 * i) * PST + base + H, PST, Xs + base * PST + base + H + 8 * j, PST, 1, 8 * i + 8, lane, acc);
-            T *o = pass == 0 ? Xs + (base + 8 * i + r) * PST + base + H + 8 * j + c : Xs + (base + H + 8 * i + r) * PST + base + 8 * j + c;
+            double *o = pass == 0 ? Xs + (base + 8 * i + r) * PST + base + H + 8 * j + c : Xs + (base + H + 8 * i + r) * PST + base + 8 * j + c;
             o[0] = pass == 0 ? acc[0] : -acc[0], o[1] = pass == 0 ? acc[1] : -acc[1];
         }
         __syncthreads();
@@ -253,9 +231,9 @@ __device__ __forceinline__ void panel_merge(const T *Ls, T *Xs, int warp, int la
 // merges without the tensor cores it took 19.5.
 // Rows and columns at or beyond the block width are the identity. The lowest failing pivot column (new numbering) goes
 // to err. Dynamic shared memory: two 64 x 66 blocks and a 64 x 9 one.
-template <typename T>
-static __global__ void __launch_bounds__(256) k_panel(Dev<T> D, const int32_t *__restrict__ fronts, int k0, int *err)
+static __global__ void __launch_bounds__(256) k_panel(Dev<double> D, const int32_t *__restrict__ fronts, int k0, int *err)
 {
+    using T = double;
     extern __shared__ __align__(16) unsigned char shp_raw[];
     T *Ls = (T *)shp_raw;      // L D below the diagonal, D on it; at the end the Cholesky factor
     T *Xs = Ls + PW * PST;     // the inverse
@@ -389,6 +367,267 @@ static __global__ void __launch_bounds__(256) k_panel(Dev<T> D, const int32_t *_
     for (int i = 0; i < 16; i++) {
         const int t = tid + 256 * i, rr = t % PW, c = t / PW;
         Inv[t] = rr < w && c < w && rr >= c ? Xs[rr * PST + c] : T(0);  // column-major
+    }
+}
+
+// Reciprocal of a pivot: the fast intrinsic as the seed and one Newton-Raphson step; pivots outside the seed's safe range
+// take a plain division.
+__device__ __forceinline__ float panel_recip(float x)
+{
+    if (!(fabsf(x) > 1e-30f && fabsf(x) < 1e30f)) return 1.0f / x;
+    const float r = __fdividef(1.0f, x);
+    return r * fmaf(-x, r, 2.0f);
+}
+
+// Recursive-doubling merge of the panel inverse at block size H: for every pair of H x H diagonal blocks,
+// X21 = -X22 (L21 X11). The upper triangles of X11 and X22 are zero, so the dot products run over whole blocks.
+template <int H>
+__device__ __forceinline__ void panel_merge_f32(float (*Ds)[PW + 1], float (*Xs)[PW + 1], float (*Ts)[33], int tid)
+{
+    constexpr int PER = H * H, TOTAL = (PW / (2 * H)) * PER, PT = TOTAL / 256;  // entries per thread: 1, 2, 4
+    float v[PT];
+#pragma unroll
+    for (int k = 0; k < PT; k++) {
+        int t = tid + 256 * k, p = t / PER, e = t % PER, i = e / H, j = e % H, b = p * 2 * H;
+        float a0 = 0, a1 = 0;
+#pragma unroll
+        for (int q = 0; q < H; q += 2) {
+            a0 = fma(Ds[b + H + i][b + q], Xs[b + q][b + j], a0);
+            a1 = fma(Ds[b + H + i][b + q + 1], Xs[b + q + 1][b + j], a1);
+        }
+        v[k] = a0 + a1;
+    }
+#pragma unroll
+    for (int k = 0; k < PT; k++) {
+        int t = tid + 256 * k, p = t / PER, e = t % PER, i = e / H, j = e % H;
+        Ts[p * H + i][j] = v[k];  // the pairs of one size fill 32 rows
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < PT; k++) {
+        int t = tid + 256 * k, p = t / PER, e = t % PER, i = e / H, j = e % H, b = p * 2 * H;
+        float a0 = 0, a1 = 0;
+#pragma unroll
+        for (int q = 0; q < H; q += 2) {
+            a0 = fma(Xs[b + H + i][b + H + q], Ts[p * H + q][j], a0);
+            a1 = fma(Xs[b + H + i][b + H + q + 1], Ts[p * H + q + 1][j], a1);
+        }
+        v[k] = a0 + a1;
+    }
+#pragma unroll
+    for (int k = 0; k < PT; k++) {
+        int t = tid + 256 * k, p = t / PER, e = t % PER, i = e / H, j = e % H, b = p * 2 * H;
+        Xs[b + H + i][b + j] = -v[k];
+    }
+    __syncthreads();
+}
+
+// Warp-level L D L^float of the eight columns J .. J + 7 of the panel block over rows J .. 63. Every lane factors the
+// 8 x 8 diagonal block in registers (no shuffles on the pivot chain), then eliminates its own rows J + 8 + lane and
+// J + 40 + lane against it. Reciprocal pivots go to rdv, the lowest failing column to *fail.
+__device__ __forceinline__ void panel_factor8_f32(float (*Ds)[PW + 1], float *rdv, int *fail, int J, int lane)
+{
+    float B[8][8], L[8][8], rd[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+        for (int j = 0; j <= i; j++) B[i][j] = Ds[J + i][J + j];
+    int bad = -1;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        if (!(B[k][k] > 0) && bad < 0) bad = k;
+        rd[k] = panel_recip(B[k][k]);
+#pragma unroll
+        for (int i = k + 1; i < 8; i++) {
+            L[i][k] = B[i][k] * rd[k];
+#pragma unroll
+            for (int j = k + 1; j <= i; j++) B[i][j] = fma(-L[i][k], B[j][k], B[i][j]);
+        }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        int r = J + 8 + lane + 32 * h;
+        if (r >= PW) continue;
+        float u[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            float v = Ds[r][J + k];
+#pragma unroll
+            for (int j = 0; j < k; j++) v = fma(-u[j], L[k][j], v);
+            u[k] = v;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) Ds[r][J + k] = u[k];
+    }
+    __syncwarp();  // every lane has read the diagonal block
+    if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+#pragma unroll
+            for (int j = 0; j <= i; j++) Ds[J + i][J + j] = B[i][j];
+            rdv[J + i] = rd[i];
+        }
+    }
+    if (lane == 0 && bad >= 0) *fail = J + bad;
+}
+
+// The same panel step in single precision, with a schedule of its own: warp 0 factors eight columns at a time over all
+// rows below them (in registers, no block barrier) while the other warps apply the previous eight to the columns beyond
+// them; the pivot columns are scaled to Cholesky form at the end, and the inverse is merged by dot products. There is no
+// FP32 MMA to shorten the products, and with them in the 8 x 8 tiles of the kernel above a panel took longer: 16.9 us
+// against 14.6 over the 60k-tet closed-die factor (B200). The order of its sums is the factor's rounding, which
+// the conjugate gradients' results follow within their tolerance. Dynamic shared memory: two 64 x 65 blocks and a
+// 32 x 33 one.
+static __global__ void __launch_bounds__(256) k_panel_f32(Dev<float> D, const int32_t *__restrict__ fronts, int k0, int *err)
+{
+    extern __shared__ __align__(16) unsigned char shp_raw[];
+    float *shp = (float *)shp_raw;
+    float (*Ds)[PW + 1] = (float (*)[PW + 1])shp;
+    float (*Xs)[PW + 1] = (float (*)[PW + 1])(shp + PW * (PW + 1));
+    float (*Ts)[33] = (float (*)[33])(shp + 2 * PW * (PW + 1));
+    __shared__ float rdv[PW];  // reciprocal pivots, then the square roots of the pivots
+    __shared__ float rsq[PW];  // reciprocal square roots of the pivots
+    __shared__ int fail;
+    int s = fronts[blockIdx.x];
+    int ms = D.m[s], w = min(PW, D.ncol[s] - k0);
+    float *F = D.F + D.front_off[s];
+    float *Inv = D.Inv + D.inv_off[s] + (int64_t)(k0 / PW) * PW * PW;
+    int tid = threadIdx.x, lane = tid & 31, r = tid & (PW - 1), cg = tid >> 6;
+    {
+        float v[16];  // all sixteen loads of a thread in flight before any store
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            int t = tid + 256 * i, rr = t % PW, c = t / PW;
+            v[i] = rr == c ? float(1) : float(0);
+            if (rr < w && c < w && rr >= c) v[i] = F[(int64_t)(k0 + c) * ms + k0 + rr];
+        }
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            int t = tid + 256 * i, rr = t % PW, c = t / PW;
+            Ds[rr][c] = v[i];
+            Xs[rr][c] = float(0);
+        }
+    }
+    if (tid == 0) fail = -1;
+    __syncthreads();
+    if (tid < 32) panel_factor8_f32(Ds, rdv, &fail, 0, lane);
+    __syncthreads();
+    // look-ahead inside the block: the CTA applies block J to the next eight columns, then warp 0 factors them
+    // while the other warps apply block J to the columns beyond; two barriers per eight columns
+    for (int J = 0; J < PW; J += 8) {
+        if (fail >= 0) {
+            if (tid == 0) atomicMin(err, D.c0[s] + k0 + fail);
+            return;  // every thread read the same flag: a uniform exit
+        }
+        if (J + 8 < PW) {
+            // the next eight columns (rows J + 8 .. 63) with block J, spread over the whole CTA
+            float v[2];
+#pragma unroll
+            for (int i = 0; i < 2; i++) {  // 8 x 56 entries at most: two per thread, loads before stores
+                int e = tid + 256 * i, c = J + 8 + (e & 7), rr = J + 8 + (e >> 3);
+                v[i] = float(0);
+                if (rr >= PW || c > rr) continue;
+                float v0 = Ds[rr][c], v1 = float(0);
+#pragma unroll
+                for (int q = 0; q < 8; q += 2) {
+                    v0 = fma(-Ds[rr][J + q] * rdv[J + q], Ds[c][J + q], v0);
+                    v1 = fma(-Ds[rr][J + q + 1] * rdv[J + q + 1], Ds[c][J + q + 1], v1);
+                }
+                v[i] = v0 + v1;
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                int e = tid + 256 * i, c = J + 8 + (e & 7), rr = J + 8 + (e >> 3);
+                if (rr < PW && c <= rr) Ds[rr][c] = v[i];
+            }
+            __syncthreads();
+        }
+        if (tid < 32) {
+            if (J + 8 < PW) panel_factor8_f32(Ds, rdv, &fail, J + 8, lane);
+        } else {
+            // columns (and rows) J + 16 .. 63: thread u keeps row J + 16 + u % 56 and walks every fourth column
+            int u = tid - 32, rr = J + 16 + u % 56, c0 = J + 16 + u / 56;
+            if (rr < PW) {
+                float lr[8], v[12];
+#pragma unroll
+                for (int q = 0; q < 8; q++) lr[q] = Ds[rr][J + q] * rdv[J + q];
+                // all loads first (at most twelve columns per thread), then the stores
+#pragma unroll
+                for (int i = 0; i < 12; i++) {
+                    int c = c0 + 4 * i;
+                    if (c > rr) break;
+                    float v0 = Ds[rr][c], v1 = float(0);
+#pragma unroll
+                    for (int q = 0; q < 8; q += 2) {
+                        v0 = fma(-lr[q], Ds[c][J + q], v0);
+                        v1 = fma(-lr[q + 1], Ds[c][J + q + 1], v1);
+                    }
+                    v[i] = v0 + v1;
+                }
+#pragma unroll
+                for (int i = 0; i < 12; i++) {
+                    int c = c0 + 4 * i;
+                    if (c > rr) break;
+                    Ds[rr][c] = v[i];
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (tid < PW) {
+        float q = sqrt(Ds[tid][tid]);
+        rdv[tid] = q;
+        rsq[tid] = float(1) / q;
+    }
+    __syncthreads();
+    {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            int c = cg + 4 * i;
+            v[i] = c == r ? rdv[r] : c < r ? Ds[r][c] * rsq[c] : float(0);
+        }
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            int c = cg + 4 * i;
+            if (c <= r) Ds[r][c] = v[i];
+        }
+    }
+    __syncthreads();
+    {
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            int t = tid + 256 * i;
+            v[i] = Ds[t % PW][t / PW];
+        }
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            int t = tid + 256 * i, rr = t % PW, c = t / PW;
+            if (rr < w && c < w && rr >= c) F[(int64_t)(k0 + c) * ms + k0 + rr] = v[i];
+        }
+    }
+    // 8x8 diagonal blocks: thread (b, j) forward-substitutes column j of block b
+    if (tid < PW) {
+        int b8 = (tid >> 3) * 8, j = tid & 7;
+        float x[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            float v = i == j ? float(1) : float(0);
+#pragma unroll
+            for (int q = 0; q < i; q++) v = fma(-Ds[b8 + i][b8 + q], x[q], v);
+            x[i] = v * rsq[b8 + i];  // 1 / L_ii
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i++) Xs[b8 + i][b8 + j] = x[i];
+    }
+    __syncthreads();
+    panel_merge_f32<8>(Ds, Xs, Ts, tid);
+    panel_merge_f32<16>(Ds, Xs, Ts, tid);
+    panel_merge_f32<32>(Ds, Xs, Ts, tid);
+    for (int t = tid; t < PW * PW; t += blockDim.x) {
+        int i = t % PW, c = t / PW;
+        Inv[t] = (i < w && c < w) ? Xs[i][c] : float(0);  // column-major, row i
     }
 }
 
@@ -1430,7 +1669,7 @@ public:
         ensure_dynamic_smem((const void *)mf::k_update_rest<T>, (int)(mf::kRestGroups * kUpdateSmem));
         if constexpr (std::is_same<T, float>::value)
             ensure_dynamic_smem((const void *)mf::k_update_sp, mf::tcu::kSmem);
-        ensure_dynamic_smem((const void *)mf::k_panel<T>, (int)kPanelSmem);
+        ensure_dynamic_smem((const void *)panel_kernel(), (int)kPanelSmem);
         ensure_dynamic_smem((const void *)mf::k_panel_trsm<T>, (int)kPairSmem);
         ensure_dynamic_smem((const void *)mf::k_xinv_gemm<T, 0>, (int)kPairSmem);
         ensure_dynamic_smem((const void *)mf::k_xinv_gemm<T, 1>, (int)kPairSmem);
@@ -1545,7 +1784,7 @@ public:
                             launch_urgent(mf::k_update<T>, dim3(prev_p1, prev_cnt), kUpdateSmem, st, dev_, fl, prev_k0,
                                           (int)mf::PW, K0 + mf::tcu::SPW, 1);
                     }
-                    launch_urgent(mf::k_panel<T>, dim3(cnt), kPanelSmem, st, dev_, fl, k0, (int *)d_err_.p);
+                    launch_urgent(panel_kernel(), dim3(cnt), kPanelSmem, st, dev_, fl, k0, (int *)d_err_.p);
                     if (maxr > 0) launch_urgent(mf::k_panel_trsm<T>, dim3(maxr, cnt), kPairSmem, st, dev_, fl, k0);
                     cuda_check(cudaEventRecord(trsm_ev_, st), "cudaEventRecord");
                     cuda_check(cudaStreamWaitEvent(ahead_, trsm_ev_, 0), "cudaStreamWaitEvent");
@@ -1804,7 +2043,13 @@ private:
     static constexpr int kChainSms = 20;
     static constexpr size_t kUpdateSmem = 2 * mf::PW * mf::SST * sizeof(T);
     static constexpr size_t kPairSmem = std::max(2 * mf::PW * mf::SST, 2 * mf::kPairBuf) * sizeof(T);
-    static constexpr size_t kPanelSmem = (2 * mf::PW * mf::PST + mf::PW * mf::PLT) * sizeof(T);
+    static constexpr size_t kPanelSmem = sizeof(T) == 8 ? (2 * mf::PW * mf::PST + mf::PW * mf::PLT) * sizeof(double)
+                                                        : (2 * mf::PW * (mf::PW + 1) + 32 * 33) * sizeof(float);
+    static auto panel_kernel()
+    {
+        if constexpr (std::is_same<T, float>::value) return mf::k_panel_f32;
+        else return mf::k_panel;
+    }
     cudaStream_t st_;
     cusolverSpHandle_t hsp_ = nullptr;
     std::vector<int64_t> inv_off_, xinv_off_;

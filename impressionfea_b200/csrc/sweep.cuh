@@ -93,30 +93,45 @@ __device__ __forceinline__ void l2_prefetch(const void *p, size_t bytes)
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global((void *)a)), "r"((uint32_t)(e - a)) : "memory");
 }
 
-// acc + sum of fa(c) fb(c) over c = first, first + G, .. < len (one lane's share of a dot product over G lanes). The
-// operands are loaded U at a time before any is used, so a lane keeps U loads in flight however short the run.
-template <int U, int G = 32, typename T, typename FA, typename FB>
-__device__ __forceinline__ T lane_dot(int first, int len, FA fa, FB fb, T acc)
+// Order of sums. In single precision a dot product is summed as VG lanes of a warp would: VG partial sums of every VG-th
+// product, added as a tree of halves (VG / 2 apart, VG / 4, .. 1). VG belongs to the front and the kind of product, not
+// to the tile: G lanes (G <= VG, as many as the tile's rows can use) hold VG / G of the partial sums each. So a solve does
+// not depend on how the tiles are cut: the single-precision factor is a preconditioner, and what its conjugate
+// gradients return within their tolerance follows the last bits of a solve. A double-precision solve is taken as
+// it is, and sums by its tile's own lanes (with fixed VG its solves measured 1 to 3 % slower).
+template <typename T>
+constexpr bool kFixedSums = sizeof(T) == 4;
+
+template <int G, int NA, typename T>
+__device__ __forceinline__ T group_sum(T (&p)[NA])
 {
-    for (int c0 = first; c0 < len; c0 += G * U) {
+#pragma unroll
+    for (int h = NA / 2; h > 0; h >>= 1)
+#pragma unroll
+        for (int k = 0; k < h; k++) p[k] += p[k + h];
+    T v = p[0];
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// Sum of fa(c) fb(c) over c = first - lane .. len - 1 (VG = 32) by eight lanes, `first` being a lane's own first entry. The
+// factor entries are loaded U at a time before any is used, so a lane keeps U loads in flight however short the run.
+template <int U, typename T, typename FA, typename FB>
+__device__ __forceinline__ T dot8(int first, int len, FA fa, FB fb)
+{
+    T p[4] = {T(0), T(0), T(0), T(0)};
+    for (int c0 = first; c0 < len; c0 += 8 * U) {
         T a[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int c = c0 + G * u;
+            const int c = c0 + 8 * u;
             a[u] = c < len ? fa(c) : T(0);
         }
 #pragma unroll
         for (int u = 0; u < U; u++)
-            if (c0 + G * u < len) acc = fma(a[u], fb(c0 + G * u), acc);
+            if (c0 + 8 * u < len) p[u % 4] = fma(a[u], fb(c0 + 8 * u), p[u % 4]);
     }
-    return acc;
-}
-template <int G, typename T>
-__device__ __forceinline__ T group_sum(T v)
-{
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+    return group_sum<8, 4>(p);
 }
 
 template <typename T>
@@ -164,49 +179,56 @@ __device__ __forceinline__ void sweep_stage(T *vs, int k0, int k1, FFetch fetch)
     }
 }
 
-// A tile: rows (or columns) [r0, r1) of the factor against an operand vector over [v0, v1) (in vs[] from v0 on); row r is
-// base[r * ld + c] for c in [lo, hi): [v0, v1), but [r, v1) for X's columns and [0, r + 1) for its rows. G lanes a row.
+// A tile: rows (or columns) [r0, r1) of the factor against an operand vector over [v0, v1) (in vs[] from v0 on). Row r holds
+// base[r * ld + c] for c in [v0, v1), but in [r, v1) for X's columns and in [0, r + 1) for its rows. Its sum has VG
+// partial sums (see above), vg of them; G lanes a row.
 template <typename T, int KIND>
 struct SweepRows {
     const T *base;
     int64_t ld;
-    int r0, r1, v0, v1;
-    // one lane's share of a batch of a row's entries: c, c + G, ...
+    int r0, r1, v0, v1, vg;
+    __device__ __forceinline__ int start(int r) const { return KIND == kSwBX ? r : v0; }
+    __device__ __forceinline__ int length(int r) const
+    {
+        return r >= r1 ? 0 : KIND == kSwBX ? v1 - r : KIND == kSwFY ? r + 1 : v1 - v0;
+    }
+    // one lane's share of a batch of a row's entries: c, c + G, ... from the row's start
     template <int G>
     __device__ __forceinline__ void load(T (&a)[kDotU<T>], int r, int c) const
     {
-        const T *p = base + (int64_t)r * ld + c;
-        const int hi = r >= r1 ? 0 : KIND == kSwFY ? r + 1 : v1;
+        const T *p = base + (int64_t)r * ld + start(r) + c;
+        const int n = length(r);
 #pragma unroll
-        for (int u = 0; u < kDotU<T>; u++)
-            a[u] = (c + G * u < hi && (KIND != kSwBX || c + G * u >= r)) ? ld_factor(p + G * u) : T(0);
+        for (int u = 0; u < kDotU<T>; u++) a[u] = c + G * u < n ? ld_factor(p + G * u) : T(0);
     }
     template <int G>
     __device__ __forceinline__ void first(T (&a)[kDotU<T>]) const
     {
         const int lane = threadIdx.x & 31;
-        load<G>(a, r0 + (threadIdx.x >> 5) * (32 / G) + lane / G, v0 + lane % G);
+        load<G>(a, r0 + (threadIdx.x >> 5) * (32 / G) + lane / G, lane % G);
     }
     // every row's dot product; a[] holds the first batch already
-    template <int G, typename FOut>
+    template <int G, int NA, typename FOut>
     __device__ __forceinline__ void dots(T (&a)[kDotU<T>], const T *vs, FOut out) const
     {
         constexpr int U = kDotU<T>, RP = 32 / G;
-        const int lane = threadIdx.x & 31, n = v1 - v0;
+        const int lane = threadIdx.x & 31;
         for (int w0 = r0 + (threadIdx.x >> 5) * RP; w0 < r1; w0 += kSwWarps * RP) {
-            const int r = w0 + lane / G;
-            if (w0 >= r0 + kSwWarps * RP) load<G>(a, r, v0 + lane % G);
-            T v = T(0);
+            const int r = w0 + lane / G, n = length(r);
+            if (w0 >= r0 + kSwWarps * RP) load<G>(a, r, lane % G);
+            T p[NA];
+#pragma unroll
+            for (int k = 0; k < NA; k++) p[k] = T(0);
             for (int c = lane % G;;) {
-                const T *x = vs + c;
+                const T *x = vs + (start(r) - v0) + c;
 #pragma unroll
                 for (int u = 0; u < U; u++)
-                    if (c + G * u < n) v = fma(a[u], x[G * u], v);
+                    if (c + G * u < n) p[u % NA] = fma(a[u], x[G * u], p[u % NA]);
                 c += G * U;
                 if (c - lane % G >= n) break;
-                load<G>(a, r, v0 + c);
+                load<G>(a, r, c);
             }
-            v = group_sum<G>(v);
+            const T v = group_sum<G, NA>(p);
             if (r < r1 && lane % G == 0) out(r, v);
         }
     }
@@ -221,9 +243,15 @@ struct SweepRows {
         else if (g == 16) first<16>(a);
         else first<32>(a);
         if (!ready()) return false;
-        if (g == 8) dots<8>(a, vs, out);
-        else if (g == 16) dots<16>(a, vs, out);
-        else dots<32>(a, vs, out);
+        const int na = vg / g;
+        if constexpr (kFixedSums<T>) {
+            if (g == 16 && na == 2) return dots<16, 2>(a, vs, out), true;
+            if (g == 8 && na == 2) return dots<8, 2>(a, vs, out), true;
+            if (g == 8 && na == 4) return dots<8, 4>(a, vs, out), true;
+        }
+        if (g == 32) dots<32, 1>(a, vs, out);
+        else if (g == 16) dots<16, 1>(a, vs, out);
+        else dots<8, 1>(a, vs, out);
         return true;
     }
 };
@@ -250,28 +278,35 @@ __device__ __forceinline__ bool sweep_small_fwd(const SweepArgs<T> &A, const Swe
         const int w = min(PW, nc - kb);
         const T *I = Inv + (int64_t)(kb / PW) * PW * PW;
         {
-            // y_blk = Linv acc_blk: four threads per row, sixteen columns each (the upper part is stored as zeros)
+            // y_blk = Linv acc_blk (VG = 32): four threads per row, every fourth column each (the upper part is
+            // stored as zeros)
             const int i = tid & 63, g = tid >> 6;
-            T f[16], v = T(0);
+            T f[16], p[8];
 #pragma unroll
-            for (int u = 0; u < 16; u++) f[u] = (i < w && 16 * g + u < w) ? ld_factor(I + (16 * g + u) * PW + i) : T(0);
+            for (int u = 0; u < 16; u++) f[u] = (i < w && g + 4 * u < w) ? ld_factor(I + (g + 4 * u) * PW + i) : T(0);
 #pragma unroll
-            for (int u = 0; u < 16; u++)
-                if (16 * g + u < w) v = fma(f[u], acc[kb + 16 * g + u], v);
-            part[tid] = v;
+            for (int u = 0; u < 8; u++) {
+                p[u] = g + 4 * u < w ? f[u] * acc[kb + g + 4 * u] : T(0);
+                if (g + 4 * u + 32 < w) p[u] = fma(f[u + 8], acc[kb + g + 4 * u + 32], p[u]);
+            }
+#pragma unroll
+            for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+                for (int k = 0; k < h; k++) p[k] += p[k + h];
+            part[tid] = p[0];
         }
         sweep_bar();
         if (tid < w) {
-            const T v = (part[tid] + part[64 + tid]) + (part[128 + tid] + part[192 + tid]);
+            const T v = (part[tid] + part[128 + tid]) + (part[64 + tid] + part[192 + tid]);
             yb[tid] = v;
             A.Y[c0 + kb + tid] = v;
         }
         sweep_bar();
-        // rows below the block, two threads a row when one pass covers them
-        const int rb = kb + w, nrow = ms - rb, H = nrow <= 128 ? 2 : 1, per = kSwCompute / H, h = tid / per;
+        // rows below the block (in double precision two threads a row when one pass covers them)
+        const int rb = kb + w, nrow = ms - rb, H = !kFixedSums<T> && nrow <= 128 ? 2 : 1, per = kSwCompute / H, h = tid / per;
         const int k0 = h * (PW / H), k1 = min(w, k0 + PW / H);
         for (int r = tid % per; r < nrow; r += per) {
-            T v = T(0);
+            T v = H == 1 ? acc[rb + r] : T(0);
             const T *col = F + (int64_t)kb * ms + rb + r;
             for (int k = k0; k < k1; k += 16) {
                 T f[16];
@@ -279,14 +314,14 @@ __device__ __forceinline__ bool sweep_small_fwd(const SweepArgs<T> &A, const Swe
                 for (int u = 0; u < 16; u++) f[u] = k + u < k1 ? ld_factor(col + (int64_t)(k + u) * ms) : T(0);
 #pragma unroll
                 for (int u = 0; u < 16; u++)
-                    if (k + u < k1) v = fma(f[u], yb[k + u], v);
+                    if (k + u < k1) v = fma(-f[u], yb[k + u], v);
             }
-            if (H == 1) acc[rb + r] -= v;
+            if (H == 1) acc[rb + r] = v;
             else part[tid] = v;
         }
         sweep_bar();
         if (H == 2) {
-            if (tid < nrow) acc[rb + tid] -= part[tid] + part[128 + tid];
+            if (tid < nrow) acc[rb + tid] += part[tid] + part[128 + tid];
             sweep_bar();
         }
     }
@@ -315,8 +350,7 @@ __device__ __forceinline__ bool sweep_small_bwd(const SweepArgs<T> &A, const Swe
         const int k = k0 + grp;
         const bool ok = k < nc;
         const T *col = F + (int64_t)(ok ? k : 0) * ms + nc;
-        T v = lane_dot<kDotU<T>, 8>(gl, ok ? nr : 0, [&](int i) { return ld_factor(col + i); }, [&](int i) { return xs[i]; }, T(0));
-        v = group_sum<8>(v);
+        const T v = dot8<kDotU<T>, T>(gl, ok ? nr : 0, [&](int i) { return ld_factor(col + i); }, [&](int i) { return xs[i]; });
         if (ok && gl == 0) acc[k] -= v;
     }
     sweep_bar();
@@ -327,8 +361,7 @@ __device__ __forceinline__ bool sweep_small_bwd(const SweepArgs<T> &A, const Swe
                 const int j = j0 + grp;
                 const bool ok = j < ke;
                 const T *col = F + (int64_t)(ok ? j : 0) * ms;
-                T v = lane_dot<kDotU<T>, 8>(ke + gl, ok ? nc : 0, [&](int k) { return ld_factor(col + k); }, [&](int k) { return acc[k]; }, T(0));
-                v = group_sum<8>(v);
+                const T v = dot8<kDotU<T>, T>(ke + gl, ok ? nc : 0, [&](int k) { return ld_factor(col + k); }, [&](int k) { return acc[k]; });
                 if (ok && gl == 0) acc[j] -= v;
             }
             sweep_bar();
@@ -338,8 +371,7 @@ __device__ __forceinline__ bool sweep_small_bwd(const SweepArgs<T> &A, const Swe
         for (int j0 = 0; j0 < w; j0 += ng) {
             const int j = j0 + grp;
             const bool ok = j < w;
-            T v = lane_dot<8, 8>((ok ? j : w) + gl, w, [&](int i) { return ld_factor(I + j * PW + i); }, [&](int i) { return acc[kb + i]; }, T(0));
-            v = group_sum<8>(v);
+            const T v = dot8<8, T>((ok ? j : w) + gl, w, [&](int i) { return ld_factor(I + j * PW + i); }, [&](int i) { return acc[kb + i]; });
             if (ok && gl == 0) xb[j] = v;
         }
         sweep_bar();
@@ -378,7 +410,7 @@ __device__ __forceinline__ bool sweep_task(const SweepArgs<T> &A, const SweepTas
     }
     case kSwFY: {
         // row r of X (read through its mirror: contiguous) against acc1
-        const SweepRows<T, kSwFY> w = {D.Xinv + t.off, nc, r0, r1, 0, r1};
+        const SweepRows<T, kSwFY> w = {D.Xinv + t.off, nc, r0, r1, 0, r1, sweep_group(nc)};
         int2 q[kSwPre];
         T b[kSwPre];
         if (t.flag)
@@ -409,7 +441,7 @@ __device__ __forceinline__ bool sweep_task(const SweepArgs<T> &A, const SweepTas
     }
     case kSwFT: {
         // row i of L21 (its mirror in the front's upper right block: contiguous) against y1
-        const SweepRows<T, kSwFT> w = {D.F + t.off + (int64_t)nc * ms, ms, r0, r1, 0, nc};
+        const SweepRows<T, kSwFT> w = {D.F + t.off + (int64_t)nc * ms, ms, r0, r1, 0, nc, sweep_group(nc)};
         const bool own = tid < r1 - r0;
         const int2 q = own ? __ldg(A.pair + t.is + nc + r0 + tid) : make_int2(-1, -1);
         T *u = D.U + t.aux;
@@ -427,7 +459,7 @@ __device__ __forceinline__ bool sweep_task(const SweepArgs<T> &A, const SweepTas
     case kSwBZ: {
         // column k of L21 against x2; the operand's place holds the entries' indices until their values are known
         const int nr = ms - nc;
-        const SweepRows<T, kSwBZ> w = {D.F + t.off + nc, ms, r0, r1, 0, nr};
+        const SweepRows<T, kSwBZ> w = {D.F + t.off + nc, ms, r0, r1, 0, nr, 32};
         const int32_t *ix = D.idx + t.is + nc;
         int *vi = reinterpret_cast<int *>(vs);
         constexpr int W = sizeof(T) / sizeof(int);
@@ -446,7 +478,7 @@ __device__ __forceinline__ bool sweep_task(const SweepArgs<T> &A, const SweepTas
     }
     default: {
         // kSwBX: column j of X against z
-        const SweepRows<T, kSwBX> w = {D.Xinv + t.off, nc, r0, r1, r0, nc};
+        const SweepRows<T, kSwBX> w = {D.Xinv + t.off, nc, r0, r1, r0, nc, sweep_group(nc)};
         return w.run(
             vs,
             [&] {
