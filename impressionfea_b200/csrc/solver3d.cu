@@ -272,7 +272,7 @@ struct Forging3D {
     int step_index = 0, warm = 0, recovery_pass = 0;
     bool have_vg_prev = false, initialized = false;
     int iterations = 0, n_fact = 0, n_pcg = 0, remesh_requests = 0, projection_reverts = 0, corner_penetrations = 0;
-    int last_cutbacks = 0, n_newton = 0, n_assemble = 0, lin_its = 0;
+    int last_cutbacks = 0, n_newton = 0, n_assemble = 0, lin_its = 0, pcg_calls = 0;
     double load = 0, reaction = 0, power = 0, last_dt = 0, rnorm = 0, beta_last = 0, max_diag = 0;
     // linear solver (SolveLinear :965-1019)
     std::unique_ptr<LinearSolver> lin;
@@ -935,6 +935,7 @@ struct Forging3D {
         int sp_grid = std::min(kReduceBlocks * 4, (topo.nn * 32 + 255) / 256);
         const PcgWork none = {nullptr, nullptr, nullptr}, W = {d_pcg_part.p, d_pcg_flag.p, d_pcg_flag.p + 1};
         const int rz[2] = {S_RZ, S_RZNEW};  // r.z of the even and odd iterations
+        pcg_calls++;
         // the residual (and |b|^2) of iteration k, copied out behind it; read one iteration later
         auto post = [&](int k) {
             cuda_check(cudaMemcpyAsync(hs.p + (1 + (k & 1)) * S_COUNT, d_scalars.p, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H scalars");
@@ -986,13 +987,21 @@ struct Forging3D {
     }
 
     // PCG iterations a reused factor may take. The reference's budget (PcgBudget, 15) in the FP64 form; in the
-    // single-precision form, whose factorisations are measured (device time) as are its PCG iterations (host
-    // time, syncs included), a reused factor is worth iterations up to pcg_budget_scale factorisations' time
-    // (at least the reference's budget, at most 120)
+    // single-precision form a reused factor is worth iterations up to pcg_budget_scale factorisations' time (at least
+    // the reference's budget, at most 120). Factorisations are measured (device time). Iterations are reckoned, not
+    // measured: a PCG call of k iterations is k + 2 solves with their products, at kPcgLevelMs a level of the elimination
+    // tree and kPcgEntryMs a million matrix entries. These are the rates (B200, 26 meshes of 3k to 200k tets, within 11 %)
+    // of the level-by-level sweeps that the scale was chosen with. Faster iterations measured by the host's clock let a
+    // factor that no longer fits be tried for longer: budgets of 54 instead of 33 at 60k tets, 95 instead of 69 at 200k,
+    // and increments of 603 ms where these rates take 376. And the velocities, which follow the
+    // tolerance of whichever solve was taken, moved with the clock.
+    static constexpr double kPcgLevelMs = 0.0193, kPcgEntryMs = 0.0424;
     int pcg_budget()
     {
         if (!pcg_early_abort || n_fact == 0 || lin_its == 0) return P.pcg_budget;
-        double f_ms = lin->factor_ms() / n_fact, it_ms = 1000.0 * t_pcg / lin_its;
+        const double f_ms = lin->factor_ms() / n_fact;
+        const double solve_ms = kPcgLevelMs * lin->symbolic().nlevels + kPcgEntryMs * 1e-6 * (double)topo.nnz;
+        const double it_ms = solve_ms * (lin_its + 2.0 * pcg_calls) / lin_its;
         if (!(f_ms > 0) || !(it_ms > 0)) return P.pcg_budget;
         return std::max(P.pcg_budget, std::min(120, (int)(pcg_budget_scale * f_ms / it_ms)));
     }
@@ -1493,7 +1502,7 @@ struct Forging3D {
         S("corner_penetrations", corner_penetrations) S("rate_ref", rate_ref) S("rate_cut", rate_cut)
         S("sig_ref", sig_ref) S("k_pen", k_pen) S("u0", u0) S("nnz", topo.nnz) S("ds_cur", ds_cur) S("warm", warm)
         S("rnorm", rnorm) S("beta", beta_last) S("max_diag", max_diag) S("have_factor", have_factor)
-        S("pcg_skip", pcg_skip) S("pcg_failures", pcg_failures) S("lin_its", lin_its) S("nbf", topo.bowner.size())
+        S("pcg_skip", pcg_skip) S("pcg_failures", pcg_failures) S("lin_its", lin_its) S("pcg_calls", pcg_calls) S("nbf", topo.bowner.size())
         S("recovery_pass", recovery_pass) S("factor_nnz", lin->factor_nonzeros()) S("max_nbr", topo.max_nbr)
         S("nn", topo.nn) S("ne", topo.ne) S("ndof", topo.ndof) S("last_dt", last_dt)
         S("t_trigger", t_trigger) S("t_prepare", t_prepare) S("t_assemble", t_assemble) S("t_linesearch", t_linesearch)
