@@ -7,6 +7,9 @@
 #include <thread>
 #include <vector>
 
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include "multifrontal.cuh"
 
 // Uploads a large pageable array: threads copy chunks into pinned slots of their own (two each) and send them on, so
@@ -14,6 +17,33 @@
 // (B200, 16 host cores), 7.2 by the driver's own staging of a pageable copy. Below kLeast starting threads takes a good
 // part of what it gains (8 MB: 0.7 ms), and memory that is pinned already is copied directly.
 class HostUpload {
+    // The calling thread's CUDA context, for the threads that copy for it: a host may run this library in a context of its
+    // own, and cudaSetDevice() would make the device's primary context current instead.
+    struct Context {
+        CUcontext ctx = nullptr;
+        PFN_cuCtxSetCurrent_v4000 set = nullptr;
+        static Context current()
+        {
+            Context c;
+            void *get = nullptr, *set = nullptr;
+            cudaDriverEntryPointQueryResult q;
+            ifea::cuda_check(cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &get, 4000, cudaEnableDefault, &q), "cuCtxGetCurrent");
+            ifea::cuda_check(cudaGetDriverEntryPointByVersion("cuCtxSetCurrent", &set, 4000, cudaEnableDefault, &q), "cuCtxSetCurrent");
+            c.set = (PFN_cuCtxSetCurrent_v4000)set;
+            if (!get || !set || ((PFN_cuCtxGetCurrent_v4000)get)(&c.ctx) != CUDA_SUCCESS)
+                throw ifea::Failure(IFEA_CUDA_ERROR, "no current CUDA context");
+            if (!c.ctx) {  // a thread that has made no CUDA call yet: the device's primary context, as for any first call
+                int dev = 0;
+                ifea::cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+                ifea::cuda_check(cudaSetDevice(dev), "cudaSetDevice");
+                if (((PFN_cuCtxGetCurrent_v4000)get)(&c.ctx) != CUDA_SUCCESS || !c.ctx)
+                    throw ifea::Failure(IFEA_CUDA_ERROR, "no current CUDA context");
+            }
+            return c;
+        }
+        cudaError_t enter() const { return set(ctx) == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue; }
+    };
+
 public:
     static constexpr size_t kLeast = 8 << 20;
     ~HostUpload() { release(); }
@@ -45,11 +75,10 @@ public:
             ifea::cuda_check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st), "cudaMemcpyAsync H2D");
             return;
         }
-        int dev = 0;
-        ifea::cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+        const Context here = Context::current();
         cudaError_t err[kThreads] = {};
         auto work = [&](int t) {
-            cudaError_t e = cudaSetDevice(dev);
+            cudaError_t e = cudaSuccess;
             int k = 0;
             for (size_t o = t * kChunk; o < bytes && e == cudaSuccess; o += kThreads * kChunk, k++) {
                 const int slot = 2 * t + (k & 1);
@@ -65,7 +94,10 @@ public:
         std::thread th[kThreads];
         for (int t = 1; t < kThreads; t++) {
             try {
-                th[t] = std::thread(work, t);
+                th[t] = std::thread([&, t] {
+                    err[t] = here.enter();
+                    if (err[t] == cudaSuccess) work(t);
+                });
             } catch (const std::exception &) {  // (no thread to be had: its chunks below)
             }
         }
