@@ -1355,6 +1355,11 @@ static __global__ void k_finite(int n, const double *x, int *flag)
 
 namespace ifea {
 
+// A wait inside a solve gave up: the solution is not to be used, the factor still is.
+struct SolveTimeout : Failure {
+    SolveTimeout() : Failure(IFEA_CUDA_ERROR, "multifrontal solve: a wait for another tile timed out") {}
+};
+
 // The linear solver behind the stepper: analyse once per pattern, factorise device values, solve on the device.
 // Implemented by the multifrontal Cholesky in double precision (the drop-in) and in single precision (the factor
 // that FP64 conjugate-gradient refinement uses as its preconditioner).
@@ -1370,6 +1375,8 @@ public:
     // x = A^-1 b; with `skip`, nothing when *skip (device) is non-zero by the time the sweep starts
     virtual void solve(const double *d_b, double *d_x, const int32_t *skip) = 0;
     virtual void check_finite(const double *d_x) = 0;
+    virtual void check_waits() = 0;  // throws SolveTimeout if a wait of an earlier solve gave up (waits for the stream)
+    virtual void set_wait_limit(double ms) = 0;  // of a solve's waits between its tiles
     virtual const MfSymbolic &symbolic() const = 0;
     virtual int64_t factor_nonzeros() const = 0;
     virtual int big_fronts() const = 0;
@@ -1464,6 +1471,7 @@ public:
         drop_graphs();
     }
     void set_profile(bool p) override { profile_ = p; }
+    void set_wait_limit(double ms) override { wait_ns_ = (uint64_t)(1e6 * ms); }
     void set_wide_rows(int m) override { wide_m_ = m; }
     int n() const { return sym_.n; }
 
@@ -1686,7 +1694,7 @@ public:
             // no more CTAs than the widest phase has tiles (and some to wait for the next one)
             sweep_grid_ = std::max(1, std::min(148 * std::max(1, per_sm), width + width / 2));
             d_cnt_.resize((size_t)mf::kCntN * S.nsuper + 2);
-            d_cnt_.zero(st_);
+            reset_waits();
         }
         cuda_check(cudaStreamSynchronize(st_), "cudaStreamSynchronize");
         analyzed_ = true;
@@ -1722,7 +1730,7 @@ public:
         float ms = 0;
         if (cudaEventElapsedTime(&ms, ev_[0], ev_[1]) == cudaSuccess) factor_ms_ += ms;
         if (e[2]) throw Failure(IFEA_CUDA_ERROR, "multifrontal factorisation: a tensor-core update timed out");
-        if (e[3]) abandoned();
+        if (e[3]) reset_waits();  // an earlier solve's, which nobody has asked about
         if (e[0] != INT_MAX) {
             int row = S.perm[e[0]];
             throw Failure(IFEA_NOT_SPD, "Stiffness matrix not positive definite at equation " + std::to_string(row) +
@@ -1978,6 +1986,7 @@ public:
         a.Z = d_y_.p + S.n;
         a.X = d_y_.p + 2 * (size_t)S.n;
         a.err = d_err_.p + 3;
+        a.wait_ns = wait_ns_;
         a.n = S.n;
         if (profile_) cuda_check(cudaEventRecord(ev_[2], st_), "cudaEventRecord");
         mf::k_sweep<T><<<sweep_grid_, mf::kSwThreads, sweep_smem_, st_>>>(a);
@@ -1998,17 +2007,29 @@ public:
         mf::k_finite<<<std::max(1, std::min((sym_.n + 255) / 256, 592)), 256, 0, st_>>>(sym_.n, d_x, d_err_.p + 1);
         cuda_check(cudaMemcpyAsync(f, d_err_.p + 1, sizeof f, cudaMemcpyDeviceToHost, st_), "D2H");
         cuda_check(cudaStreamSynchronize(st_), "cudaStreamSynchronize");
-        if (f[2]) abandoned();
+        if (f[2]) gave_up();
         if (f[0]) throw Failure(IFEA_NOT_SPD, "Stiffness matrix not positive definite at equation -1 (pivot NaN).");
     }
 
-private:
-    // a sweep gave up waiting: its counters are not usable any more
-    void abandoned()
+    void check_waits() override
     {
-        d_err_.zero(st_);
+        int32_t e = 0;
+        cuda_check(cudaMemcpyAsync(&e, d_err_.p + 3, sizeof e, cudaMemcpyDeviceToHost, st_), "D2H");
+        cuda_check(cudaStreamSynchronize(st_), "cudaStreamSynchronize");
+        if (e) gave_up();
+    }
+
+private:
+    // a solve that gave up waiting leaves counters that are not usable any more
+    void reset_waits()
+    {
+        cuda_check(cudaMemsetAsync(d_err_.p + 3, 0, sizeof(int32_t), st_), "cudaMemsetAsync");
         d_cnt_.zero(st_);
-        throw Failure(IFEA_CUDA_ERROR, "multifrontal solve: a wait for another tile timed out");
+    }
+    void gave_up()
+    {
+        reset_waits();
+        throw SolveTimeout();
     }
     void drop_graphs()
     {
@@ -2020,6 +2041,7 @@ private:
     double factor_ms_ = 0, solve_ms_ = 0, setup_s_[4] = {0, 0, 0, 0};
     int64_t n_solves_ = 0;
     bool profile_ = false;
+    uint64_t wait_ns_ = 2000000000;
     int wide_m_ = mf::kWideM;
     bool use_tc_ = std::is_same<T, float>::value;  // tensor-core trailing updates (single precision)
     int64_t tc_launches_ = 0;                        // tensor-core update launches per factorisation

@@ -311,6 +311,7 @@ struct Forging3D {
     double pcg_forcing = 0;
     double lin_tol = 1e-7;  // the PCG tolerance of the linear solve in progress
     int factor_step = -1, stale_failures = 0;  // increment of the cached factor; failed tries of a stale one
+    double solve_wait_ms = 2000;  // limit of a solve's waits between its tiles
     int wide_rows = mf::kWideM;  // fronts at least this tall use the multi-CTA solve path
     // learned warm start: mode bit 1 records (inputs, target) of every accepted increment into the network's
     // training set, bit 2 starts each increment from the network's prediction when its energy is lower than
@@ -422,6 +423,7 @@ struct Forging3D {
         else
             lin.reset(new MfSolverT<double>(st));
         lin->set_wide_rows(wide_rows);
+        lin->set_wait_limit(solve_wait_ms);
         need_analyze = true;
         have_factor = false;
         pcg_skip = pcg_failures = 0;
@@ -965,6 +967,8 @@ struct Forging3D {
             cuda_check(cudaEventSynchronize(pcg_ev[it & 1]), "cudaEventSynchronize");
             const double *h = hs.p + (1 + (it & 1)) * S_COUNT;
             const double rr = h[S_RR];
+            // (a solve that was given up has NaN in its solution)
+            if (!std::isfinite(rr)) lin->check_waits();
             if (it == 0) {
                 r0 = sqrt(rr);
                 bnorm = sqrt(h[S_BB]);
@@ -1052,6 +1056,9 @@ struct Forging3D {
                 lin->solve(b, x, nullptr);
                 lin->check_finite(x);
             }
+        } catch (SolveTimeout &) {
+            have_factor = false;
+            throw;
         } catch (Failure &f) {
             have_factor = false;
             if (f.status == IFEA_NOT_SPD) throw;
@@ -1244,6 +1251,7 @@ struct Forging3D {
         cudaEventDestroy(b);
         have_factor = true;
         factor_step = step_index;
+        lin->check_waits();
         return ms;
     }
 
@@ -1514,7 +1522,7 @@ struct Forging3D {
         S("factor_fp32", lin->value_bytes() == 4) S("fp32_fallbacks", fp32_fallbacks) S("refine_its", refine_its)
         S("pcg_early_abort", pcg_early_abort) S("pcg_failures_total", pcg_failures_total) S("wide_front_rows", wide_rows) S("tc_updates", lin->tc_launches())
         S("factor_gflop", factor_gflop())
-        S("pcg_budget_now", pcg_budget()) S("pcg_budget_scale", pcg_budget_scale) S("pcg_forcing", pcg_forcing)
+        S("solve_wait_ms", solve_wait_ms) S("pcg_budget_now", pcg_budget()) S("pcg_budget_scale", pcg_budget_scale) S("pcg_forcing", pcg_forcing)
         S("ws_used", ws_used) S("ws_fallbacks", ws_fallbacks) S("ws_mode", ws_mode) S("ws_policy", ws_policy) S("ws_smooth", ws_smooth)
         S("ws_last_step", ws_last_step)
         S("remesh", remesh_enabled) S("remesh_count", remesh_count) S("remesh_rejected", remesh_rejected)
@@ -1532,6 +1540,11 @@ struct Forging3D {
         else if (nm == "ds_cur") ds_cur = v;
         else if (nm == "warm") warm = (int)v;
         else if (nm == "profile_solves") lin->set_profile(v != 0);
+        else if (nm == "solve_wait_ms") {
+            if (!(v >= 0 && v <= 1e6)) throw Failure(IFEA_INPUT_INVALID, "solve_wait_ms must lie in [0, 1e6]");
+            solve_wait_ms = v;
+            lin->set_wait_limit(v);
+        }
         else if (nm == "tc_update") lin->set_tc(v != 0, 1024);
         else if (nm == "tc_rows") lin->set_tc(true, (int)v);
         else if (nm == "wide_front_rows") {

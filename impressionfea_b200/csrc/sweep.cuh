@@ -12,10 +12,11 @@
 // hand-over costs a CTA about half a microsecond, which plain loads of 24 or more warps hide.)
 //
 // Progress needs no co-residency: tickets are drawn in list order by running CTAs, so the lowest unfinished task
-// always has its inputs complete. Every wait is bounded all the same (two seconds); one that gives up sets a sticky
-// error word and the solution to NaN, and every CTA leaves. Counters are monotonic over the solves of an analysis
-// (targets scale with the solve's number), so nothing is cleared between solves. Every sum has a fixed order:
-// solves are bit-reproducible.
+// always has its inputs complete. Every wait is bounded all the same (two seconds unless the host sets another limit);
+// one that gives up sets a sticky error word, every CTA leaves, and what was not computed of the solution is NaN (tasks
+// still at work may store their part of it). The host clears the word with the counters when it reads it. Counters
+// are monotonic over the solves of an analysis (targets scale with the solve's number), so nothing is cleared between
+// solves. Every sum has a fixed order: solves are bit-reproducible.
 //
 // What bounds it: the bytes of the factor on the large levels (3.3 TB/s over a whole solve of 308 M FP32 entries),
 // the chain of dependent phases towards the root on small factors (two going up and two coming down per level, each
@@ -148,6 +149,7 @@ struct SweepArgs {
     double *x;
     T *A1, *Y, *Z, *X;  // assembled right-hand sides (per front row); y, z and x in the new numbering
     int *err;
+    uint64_t wait_ns;   // a wait's limit; zero: a counter is looked at once
     int n;
 };
 
@@ -522,8 +524,8 @@ __device__ __forceinline__ void sweep_prefetch(const Dev<T> &D, const SweepTask 
     }
 }
 
-// Bounded wait until a counter has reached its target: false when another CTA gave up or two seconds have passed.
-__device__ __forceinline__ bool sweep_poll(const uint32_t *c, uint32_t target, const int *err)
+// Bounded wait until a counter has reached its target: false when another CTA gave up or the limit has passed.
+__device__ __forceinline__ bool sweep_poll(const uint32_t *c, uint32_t target, uint64_t wait_ns, const int *err)
 {
     uint64_t t0 = 0;
     for (uint32_t it = 0;; it++) {
@@ -534,11 +536,12 @@ __device__ __forceinline__ bool sweep_poll(const uint32_t *c, uint32_t target, c
             asm volatile("fence.acq_rel.gpu;" ::: "memory");
             return true;
         }
+        if (wait_ns == 0) return false;
         if ((it & 255) == 255) {
             uint64_t now;
             asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
             if (t0 == 0) t0 = now;
-            if (now - t0 > 2000000000ull || *(volatile const int *)err) return false;
+            if (now - t0 > wait_ns || *(volatile const int *)err) return false;
         }
     }
 }
@@ -578,7 +581,7 @@ static __global__ void __launch_bounds__(kSwThreads, kSwCtas) k_sweep(const Swee
             int ok = 1;
             if (lane == 0) {
                 const int w = desc[p].wait;
-                ok = w < 0 || sweep_poll(A.cnt + w, solves * (uint32_t)desc[p].target, A.err);
+                ok = w < 0 || sweep_poll(A.cnt + w, solves * (uint32_t)desc[p].target, A.wait_ns, A.err);
                 if (!ok) atomicExch(A.err, 1);
                 go[p] = ok;
             }
