@@ -5,11 +5,12 @@
 // factorisation assembles the matrix values into the fronts of a level (one gather), adds the children's update
 // matrices (extend-add, one launch per child rank so every entry sums its children in a fixed order), then
 // eliminates the supernode's pivot columns in panels of 64: a one-CTA-per-front kernel factors the panel's
-// diagonal block in shared memory and solves the rows below it, and a tiled kernel subtracts the panel's
-// outer product from the trailing front. What remains in the trailing block is the update matrix the parent
-// reads; the pivot columns are the factor, so no copy is made. Products are accumulated with explicit fused
-// multiply-adds (the library is built without contraction, which the element kernels' parity needs). The solves walk the levels up (update vectors)
-// and down (gathers from solved ancestors). Nothing uses atomics on values: results are bit-reproducible.
+// diagonal block in shared memory and inverts it, a tiled kernel multiplies the rows below it by that inverse, and
+// tiled kernels subtract the products from the trailing front, inside a super-panel of 256 columns panel by panel, right of
+// it once for all. What remains in the trailing block is the update matrix the parent reads; the pivot columns are
+// the factor, so no copy is made. Products are accumulated with explicit fused multiply-adds or on the tensor cores (the
+// library is built without contraction, which the element kernels' parity needs). The solves are one persistent
+// kernel over a list of tile tasks (sweep.cuh). Nothing uses atomics on values: results are bit-reproducible.
 #pragma once
 #include <cusolverSp.h>
 #include <cusparse.h>
@@ -36,7 +37,7 @@ constexpr int KST = KC + 4;  // row stride of an operand tile held by columns, K
 
 template <typename T>
 struct Dev {
-    const int32_t *ncol, *m, *c0, *idx_start, *idx, *relmap_start, *relmap, *uvec_start;
+    const int32_t *ncol, *m, *c0, *idx_start, *idx, *relmap_start, *relmap;
     const int32_t *gat_src;  // the children's update-vector entries that land on a front row (lists of three or more)
     const int64_t *front_off, *inv_off, *xinv_off;
     T *F, *U, *Inv, *Xinv;
@@ -1390,7 +1391,8 @@ public:
     virtual int value_bytes() const = 0;
     virtual int64_t tc_launches() const = 0;  // tensor-core trailing-update launches in one factorisation
     virtual void set_tc(bool on, int rows) = 0;  // tensor-core trailing updates (single precision) from `rows` rows
-    // host seconds spent in: 0 symbolic analysis, 1 its device tables, 2 the factorisation graph, 3 unused
+    // host seconds spent in: 0 symbolic analysis, 1 its device tables, 2 the factorisation graph, 3 nothing any more (a
+    // solve needs no graph; the scalar t_graph_solve that reads it stays)
     virtual double setup_s(int part) const = 0;
 };
 
@@ -1509,7 +1511,7 @@ public:
 
         d_ncol_.upload(S.ncol, st_); d_m_.upload(S.m, st_); d_c0_.upload(S.c0, st_); d_idxs_.upload(S.idx_start, st_);
         d_idx_.upload(S.idx, st_); d_rms_.upload(S.relmap_start, st_); d_rm_.upload(S.relmap, st_);
-        d_uvs_.upload(S.uvec_start, st_); d_off_.upload(S.front_off, st_); d_par_.upload(S.parent, st_);
+        d_off_.upload(S.front_off, st_); d_par_.upload(S.parent, st_);
         d_perm_.upload(S.perm, st_); d_adst_.upload(S.a_dst.data(), S.a_dst.size(), st_);
         d_asrc_.upload(S.a_src.data(), S.a_src.size(), st_);
         d_ext_.upload(S.ext_child, st_);
@@ -1661,7 +1663,6 @@ public:
         for (auto &e : fork_ev_) cuda_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         d_xinv_w_.resize(std::max<int64_t>(max_slots * mf::PW * mf::PW, 1));
         d_xinv_tasks_.upload(tasks, st_);
-        d_small_.upload(small_list_, st_);
         d_xinv_off_.upload(xinv_off_, st_);
         d_Xinv_.resize(std::max<int64_t>(xinv_total, 1));
         d_Abig_.resize(S.idx_start[S.nsuper]);
@@ -1669,7 +1670,7 @@ public:
         d_U_.resize(std::max<int64_t>(S.uvec_pool, 1));
         d_y_.resize(3 * (size_t)S.n);
         dev_.ncol = d_ncol_; dev_.m = d_m_; dev_.c0 = d_c0_; dev_.idx_start = d_idxs_; dev_.idx = d_idx_;
-        dev_.relmap_start = d_rms_; dev_.relmap = d_rm_; dev_.uvec_start = d_uvs_; dev_.front_off = d_off_; dev_.F = d_F_; dev_.U = d_U_;
+        dev_.relmap_start = d_rms_; dev_.relmap = d_rm_; dev_.front_off = d_off_; dev_.F = d_F_; dev_.U = d_U_;
         dev_.gat_src = d_gsrc_;
         dev_.inv_off = d_inv_off_; dev_.Inv = d_Inv_; dev_.xinv_off = d_xinv_off_; dev_.Xinv = d_Xinv_;
         ensure_dynamic_smem((const void *)mf::k_update<T>, (int)kUpdateSmem);
@@ -2087,14 +2088,14 @@ private:
     DBuf<int64_t> d_inv_off_, d_xinv_off_;
     DBuf<int64_t> d_mirror_ts_;   // the wide fronts' mirror tiles, prefix per front
     int64_t mirror_tiles_ = 0;
-    DBuf<int32_t> d_small_, d_big_, d_gsrc_;
+    DBuf<int32_t> d_big_, d_gsrc_;
     DBuf<int2> d_pair_;
     DBuf<T> d_Inv_, d_Xinv_, d_Abig_;
     cusparseMatDescr_t descr_ = nullptr;
     MfSymbolic sym_;
     bool analyzed_ = false, factored_ = false;
     std::vector<int32_t> lvl_sorted_;
-    DBuf<int32_t> d_ncol_, d_m_, d_c0_, d_idxs_, d_idx_, d_rms_, d_rm_, d_uvs_, d_par_, d_perm_, d_asrc_, d_ext_, d_lvl_, d_err_;
+    DBuf<int32_t> d_ncol_, d_m_, d_c0_, d_idxs_, d_idx_, d_rms_, d_rm_, d_par_, d_perm_, d_asrc_, d_ext_, d_lvl_, d_err_;
     DBuf<int64_t> d_off_, d_adst_;
     DBuf<T> d_F_, d_U_, d_y_;
     mf::Dev<T> dev_{};

@@ -42,14 +42,16 @@ enum SweepKind : int32_t {
 
 // Everything a task needs to address its data, so that nothing is looked up once its inputs are complete.
 struct __align__(16) SweepTask {
-    int32_t kind, s, r0, r1;
+    int32_t kind, flag, r0, r1;
     int32_t wait, target;  // counter and its value per solve (wait < 0: none)
-    int32_t done, flag;    // counter to raise (< 0: none)
-    int32_t nc, ms, c0, is;  // pivots, rows, first pivot (new numbering), first entry in the per-row arrays
+    int32_t done;          // counter to raise (< 0: none)
+    int32_t is;            // first entry in the per-row arrays
+    int32_t nc, ms, c0;    // pivots, rows, first pivot (new numbering)
     int64_t off;             // the front (small fronts, kSwFT, kSwBZ) or its pivot-block inverse (kSwFY, kSwBX)
     int64_t aux;             // the update vector (kSwFT, kSwFS); the panel inverses (kSwBS)
-    int64_t inv, pad;        // the panel inverses (kSwFS)
+    int64_t inv;             // the panel inverses (kSwFS)
 };
+static_assert(sizeof(SweepTask) % 16 == 0, "tasks are read 16 bytes at a time");
 
 constexpr int kSwCtas = 4;                    // CTAs per SM (three or two measured the same or slower)
 constexpr int kSwWarps = 8;                   // computing warps
@@ -661,7 +663,7 @@ inline void sweep_tasks(const MfSymbolic &S, const std::vector<int32_t> &small_s
     };
     auto add = [&](SweepKind kind, int s, int r0, int r1, int wait, int target, int done, int flag) {
         SweepTask t = {};
-        t.kind = kind, t.s = s, t.r0 = r0, t.r1 = r1, t.wait = target ? wait : -1, t.target = target, t.done = done, t.flag = flag;
+        t.kind = kind, t.r0 = r0, t.r1 = r1, t.wait = target ? wait : -1, t.target = target, t.done = done, t.flag = flag;
         t.nc = S.ncol[s], t.ms = S.m[s], t.c0 = S.c0[s], t.is = S.idx_start[s];
         t.off = kind == kSwFY || kind == kSwBX ? xinv_off[s] : S.front_off[s];
         t.aux = kind == kSwBS ? inv_off[s] : S.uvec_start[s];

@@ -69,7 +69,6 @@ class WarmStartNet {
     DBuf<float> dx_, dt_;
     int64_t count_ = 0, cap_ = 0;
     std::vector<float> norm_host_;
-    HostPinned<float> hloss_;
 };
 
 }  // namespace ifea
