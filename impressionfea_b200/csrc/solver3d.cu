@@ -992,20 +992,25 @@ struct Forging3D {
 
     // PCG iterations a reused factor may take. The reference's budget (PcgBudget, 15) in the FP64 form; in the
     // single-precision form a reused factor is worth iterations up to pcg_budget_scale factorisations' time (at least
-    // the reference's budget, at most 120). Factorisations are measured (device time). Iterations are reckoned, not
-    // measured: a PCG call of k iterations is k + 2 solves with their products, at kPcgLevelMs a level of the elimination
-    // tree and kPcgEntryMs a million matrix entries. These are the rates (B200, 26 meshes of 3k to 200k tets, within 11 %)
-    // of the level-by-level sweeps that the scale was chosen with. Faster iterations measured by the host's clock let a
-    // factor that no longer fits be tried for longer: budgets of 54 instead of 33 at 60k tets, 95 instead of 69 at 200k,
-    // and increments of 603 ms where these rates take 376. And the velocities, which follow the
-    // tolerance of whichever solve was taken, moved with the clock.
-    static constexpr double kPcgLevelMs = 0.0193, kPcgEntryMs = 0.0424;
+    // the reference's budget, at most 120). Factorisations are measured (device time). Iterations are reckoned from the
+    // analysis, at the rates of the level-by-level sweeps that the scale was chosen with (B200, 26 meshes of 6k to 200k
+    // tets, within 4 %; with them a factorisation took 3 % longer, which the rates leave out): a PCG call of k
+    // iterations is k + 2 solves with their products; a solve a time per level of the elimination tree, more once the
+    // factor no longer stays in L2 between solves, and a time per factor entry; a context's first solve its capture.
+    // Iterations measured by the host's clock let a factor that no longer fits be tried for longer as they got faster:
+    // budgets of 54 instead of 33 at 60k tets, 95 instead of 69 at 200k, and increments of 603 ms where these rates take
+    // 373. And the velocities, which follow the tolerance of whichever solve was taken, moved with the clock.
+    static constexpr double kPcgLevelMs = 0.0209, kPcgColdMs = 0.0091, kPcgEntryMs = 2.25e-9, kPcgFirstMs = 0.25;
+    double reckoned_solve_ms() const
+    {
+        const double nnz = (double)lin->factor_nonzeros(), cold = rclamp((nnz - 5e6) / 7e6, 0, 1);
+        return lin->symbolic().nlevels * (kPcgLevelMs + cold * kPcgColdMs) + nnz * kPcgEntryMs;
+    }
     int pcg_budget()
     {
         if (!pcg_early_abort || n_fact == 0 || lin_its == 0) return P.pcg_budget;
         const double f_ms = lin->factor_ms() / n_fact;
-        const double solve_ms = kPcgLevelMs * lin->symbolic().nlevels + kPcgEntryMs * 1e-6 * (double)topo.nnz;
-        const double it_ms = solve_ms * (lin_its + 2.0 * pcg_calls) / lin_its;
+        const double it_ms = (reckoned_solve_ms() * (lin_its + 2.0 * pcg_calls) + kPcgFirstMs) / lin_its;
         if (!(f_ms > 0) || !(it_ms > 0)) return P.pcg_budget;
         return std::max(P.pcg_budget, std::min(120, (int)(pcg_budget_scale * f_ms / it_ms)));
     }
