@@ -492,7 +492,7 @@ __device__ __forceinline__ bool friction_node(const View3 &V, int n, const doubl
     return true;
 }
 
-constexpr int kColumnWarps = 10;  // warps of a block, at most
+constexpr int kColumnWarps = 8;  // warps of a block, at most
 
 // Column-node assembly, one warp per node j:
 //   R_j = (K_vol v)_j + sum over tets of j in ascending order of the rotated element residual + friction;
@@ -501,9 +501,9 @@ constexpr int kColumnWarps = 10;  // warps of a block, at most
 //
 // Latency bounds it: a node is some 25 tets and 60 neighbours, all looked up through lists. So what a node needs is
 // loaded before it is used (neighbours four loads ahead, the residuals of ten tets at once, K_vol read once for product
-// and chunk), a block's nine additions are read, added and written together, and as many warps run as the chunks
-// leave room for (B200, 200k tets: 250 us; one look-up after another, and with the element products over zero
-// terms and by components known at run time only, 760).
+// and chunk), and a block's nine additions are read, added and written together (B200, 200k tets: 246 us; one look-up
+// after another, and with the element products over zero terms and by components known at run time only, 760). Eight
+// warps a block: the energies' partial sums are theirs (ten, for which there was room, took 256 us).
 template <int MODE, bool BC>
 __global__ void __launch_bounds__(kColumnWarps * 32, 2) k_columns(View3 V, const double *__restrict__ v, int newton, int max_nbr)
 {
@@ -1164,8 +1164,8 @@ __global__ void k_initial_velocity(View3 V, double rate_ref, double cx, double c
 
 namespace ifea {
 // PCG pieces with the step scalars and the convergence test kept on the device (Pcg, Forging3DSolver.cs:1051-1087):
-// five launches an iteration (product and p.q; x, r and |r|^2; the factor's solve; r.z; p) where the dot products, their
-// final sums and the roll of r.z took ten, and nothing of an iteration does anything once *stop is set, so the host
+// five launches an iteration (product and p.q; x, r and |r|^2; the factor's solve; r.z; p; in the single-precision form six,
+// p.q on its own) where the dot products, their final sums and the roll of r.z took ten, and nothing of an iteration does anything once *stop is set, so the host
 // may run one iteration ahead of the residual it reads. The launches are bound by their own fixed cost (2-3 us each
 // at 5k-30k tets).
 // r = b - q (q = A x), or x += alpha p, r -= alpha q; then scalars[S_RR] = r.r and whether the iteration has converged.
@@ -1200,7 +1200,7 @@ __global__ void k_pcg_xr(View3 V, double tol, int slot_rz, double *x, double *r,
         *W.stop = sqrt(rr[0]) <= tol * sqrt(V.scalars[S_BB]);
     }
 }
-__global__ void k_pcg_rz(View3 V, int slot, const double *r, const double *z, PcgWork W)
+__global__ void k_pcg_dot(View3 V, int slot, const double *r, const double *z, PcgWork W)
 {
     if (*W.stop) return;
     double rz[1] = {0};

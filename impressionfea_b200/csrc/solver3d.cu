@@ -362,7 +362,7 @@ struct Forging3D {
     DBuf<double> d_pcg_part;         // partial sums of a PCG kernel
     DBuf<int32_t> d_pcg_flag;        // its arrival ticket, the convergence flag
     HostPinned<int32_t> hi;
-    int wpb = 8;          // warps per block of the column kernels
+    int wpb = 8, kvol_wpb = 10;  // warps per block of the column kernels, of k_kvol
     size_t col_smem = 0;  // dynamic shared memory of the column kernels
     int max_ring = 1;     // most nodes around one, itself among them
     int ring_warps() const { return std::max(1, std::min(8, 160 * 1024 / (24 * max_ring))); }
@@ -658,8 +658,8 @@ struct Forging3D {
         d_elrate.zero(st);
         // column-kernel launch shape: chunk of 9*max_nbr doubles per warp in shared memory
         size_t per_warp = 9 * (size_t)topo.max_nbr * sizeof(double);
-        // (two blocks an SM where ten warps' chunks, or fewer, leave room for them)
-        wpb = (int)std::max<size_t>(1, std::min<size_t>(kColumnWarps, (112 * 1024) / std::max<size_t>(per_warp, 1)));
+        // (the energies are summed by these warps: their number is part of the sums' order)
+        wpb = (int)std::max<size_t>(1, std::min<size_t>(kColumnWarps, (160 * 1024) / std::max<size_t>(per_warp, 1)));
         col_smem = per_warp * wpb;
         if (per_warp > 200 * 1024) throw Failure(IFEA_INPUT_INVALID, "node neighbourhood too large for the column kernel");
         auto set_smem = [&](const void *f) {
@@ -669,7 +669,10 @@ struct Forging3D {
         set_smem((const void *)k_columns<ASM_MATRIX, false>);
         set_smem((const void *)k_columns<ASM_RESIDUAL, false>);
         set_smem((const void *)k_columns<ASM_ENERGY, false>);
-        set_smem((const void *)k_kvol);
+        // (k_kvol sums nothing over its block: ten warps, two blocks an SM, where the chunks leave room; 163 us at 200k tets,
+        // 176 with the eight of k_columns)
+        kvol_wpb = (int)std::max<size_t>(1, std::min<size_t>(10, (112 * 1024) / std::max<size_t>(per_warp, 1)));
+        ensure_dynamic_smem((const void *)k_kvol, (int)(per_warp * kvol_wpb));
         max_ring = 1;
         for (int n = 0; n < topo.nn; n++) max_ring = std::max(max_ring, topo.g_start[n + 1] - topo.g_start[n]);
         ensure_dynamic_smem((const void *)k_anp_coef, ring_warps() * 3 * max_ring * (int)sizeof(double));
@@ -795,7 +798,7 @@ struct Forging3D {
         k_anp_coef<<<std::min(8 * 148, (topo.nn + rw - 1) / rw), rw * 32, rw * 3 * max_ring * sizeof(double), st>>>(V, max_ring);
         int G = (int)topo.g_node.size();
         k_clocal<<<grid(G), 256, 0, st>>>(V, G);
-        k_kvol<<<std::min(kReduceBlocks * 2, (topo.nn + wpb - 1) / wpb), wpb * 32, col_smem, st>>>(V, topo.max_nbr);
+        k_kvol<<<std::min(kReduceBlocks * 2, (topo.nn + kvol_wpb - 1) / kvol_wpb), kvol_wpb * 32, col_smem / wpb * kvol_wpb, st>>>(V, topo.max_nbr);
         k_friction_prep<<<grid(topo.nn), 256, 0, st>>>(V);
         int trend = P.extrapolate_start && warm && have_vg_prev;
         k_guess<<<grid(topo.nn), 256, 0, st>>>(V, trend);
@@ -938,6 +941,10 @@ struct Forging3D {
         const PcgWork none = {nullptr, nullptr, nullptr}, W = {d_pcg_part.p, d_pcg_flag.p, d_pcg_flag.p + 1};
         const int rz[2] = {S_RZ, S_RZNEW};  // r.z of the even and odd iterations
         pcg_calls++;
+        // In the single-precision form p.q is summed over the entries, as the other dot products are, by a launch of its own
+        // (2 us of an iteration's 150 to 900), not over the product's rows: with sums in that other order velocities that
+        // end unconverged were 3e-9 of their size away.
+        const bool own_pq = lin->value_bytes() == 4;
         // the residual (and |b|^2) of iteration k, copied out behind it; read one iteration later
         auto post = [&](int k) {
             cuda_check(cudaMemcpyAsync(hs.p + (1 + (k & 1)) * S_COUNT, d_scalars.p, S_COUNT * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H scalars");
@@ -945,7 +952,7 @@ struct Forging3D {
         };
         auto solve_z = [&](int slot) {
             lin->solve(d_pr, d_pz, W.stop);
-            k_pcg_rz<<<kReduceBlocks, 256, 0, st>>>(V, slot, d_pr, d_pz, W);
+            k_pcg_dot<<<kReduceBlocks, 256, 0, st>>>(V, slot, d_pr, d_pz, W);
         };
         k_dot2<<<kReduceBlocks, 256, 0, st>>>(V, b, b, S_BB, nullptr, 0);
         finalize({S_BB});
@@ -958,7 +965,8 @@ struct Forging3D {
         double r0 = 0, bnorm = 0;
         for (int it = 0;; it++) {
             if (it < max_it) {  // iteration `it`, before its starting residual is known here (the device knows it)
-                k_spmv<<<sp_grid, 256, 0, st>>>(V, d_pp, d_pq, W);
+                k_spmv<<<sp_grid, 256, 0, st>>>(V, d_pp, d_pq, own_pq ? PcgWork{nullptr, nullptr, W.stop} : W);
+                if (own_pq) k_pcg_dot<<<kReduceBlocks, 256, 0, st>>>(V, S_PQ, d_pp, d_pq, W);
                 k_pcg_xr<<<kReduceBlocks, 256, 0, st>>>(V, tol, rz[it & 1], x, d_pr, d_pp, d_pq, W);
                 post(it + 1);
                 solve_z(rz[(it + 1) & 1]);
