@@ -43,10 +43,12 @@ struct Dev {
     T *F, *U, *Inv, *Xinv;
 };
 
-// Fronts at least this tall (and with more than kWideMinCols pivot columns) get a full pivot-block inverse and
-// multi-CTA solves; the others are eliminated by one CTA each. Sending the narrow tall fronts (two panels or less)
-// to the one-CTA path as well measured slower on the closed-die factor (1.77 against 1.46 ms per solve), so the
-// column bound is off.
+// Fronts at least this tall (and with more than kWideMinCols pivot columns) get a full pivot-block inverse and are solved
+// in tiles; the others are eliminated by one CTA each. Solve times (B200, ms) with the height at 96 / 192 / 256 / 384 / 1000:
+// 5k tets FP64 0.104 / 0.102 / 0.096 / 0.101 / 0.35, 32k FP64 0.244 / 0.244 / 0.240 / 0.238 / 0.41, 60k FP32 0.288 / 0.285 /
+// 0.283 / 0.284 / 0.41, 200k FP32 0.760 / 0.756 / 0.754 / 0.756 / 0.86: flat around 192, which stays (a front's form is
+// part of its sums' order). Narrow tall fronts on one CTA as well, at most 64 or 128 pivot columns: 32k FP64 0.285 and 0.372
+// instead of 0.244, 200k FP32 0.793 and 1.01 instead of 0.756, so the column bound is off.
 constexpr int kWideM = 192;
 constexpr int kWideMinCols = 0;
 
